@@ -71,7 +71,8 @@ typedef struct {
   int32_t tile_variant;  /* tile kernel: 0 auto, 1 table-driven, 2 register-resident prefetch,
                             3 staged asynchronous copies                                        */
   int32_t ragged;        /* staged tile kernel's ragged tiles (last blocks of dimensions that
-                            the tile does not divide): 0 = planned as transpositions of their
+                            the tile does not divide): 0 = moved within the staged kernel's own
+                            launch where they are few, else planned as transpositions of their
                             own and moved by the staged kernel, 1 = element-wise kernel         */
   /* loop_order == 4: TTC's loop order (--loopPerm, GPUtransposeGenerator.py:203-230), the caller's
      dimensions from the fastest-varying tile index to the slowest, packed 4 bits per dimension as
@@ -84,8 +85,8 @@ typedef struct {
                             copies in flight); 0 = planner's choice                             */
   int32_t ctas_per_sm;   /* staged tile kernel: resident CTAs per SM (1..8, capped by what fits);
                             0 = planner's choice. `blocks`, when set, takes precedence          */
-  int32_t round_robin;   /* staged tile kernel: 0 = planner's choice (claims for tiles of 16 KiB
-                            or more when every CTA has 16 or more), 1 = fixed round-robin order
+  int32_t round_robin;   /* staged tile kernel: 0 = planner's choice (claims for calls that move
+                            128 MB or more, 150 MB with beta, with 8 or more tiles per CTA), 1 = fixed round-robin order
                             (tile blockIdx + k * CTAs), -1 = CTAs claim tiles in order from
                             counters the plan owns                                              */
   int32_t shifted_runs;  /* staged tile kernel: 1 = copy A runs that 16-byte accesses cannot
@@ -100,7 +101,9 @@ typedef struct {
                             planner's model finds fewer bank conflicts in the gather that way;
                             0 or -1 = a warp takes 32 consecutive B vectors                     */
   int32_t claim_group;   /* staged tile kernel with claimed tiles: consecutive tiles per claim
-                            (1..64); 0 = planner's choice (2)                                   */
+                            (1..8; more counts as 8); 0 = planner's choice (4 for tiles under
+                            13 KiB, 1 for tiles of 20 KiB or more in three stages with B runs
+                            of at most 160 bytes, else 2)                                       */
 } ttcb_tuning;
 
 typedef struct ttcb_plan ttcb_plan;

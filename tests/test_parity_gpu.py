@@ -337,6 +337,26 @@ def test_edge_plans_random_ragged_problems(offset):
     assert with_edges >= 12, with_edges
 
 
+@pytest.mark.parametrize("dtype,beta", [("s", 0.0), ("s", -0.5), ("d", 0.0), ("d", -0.5), ("c", 1.2), ("zc", 0.0),
+                                        ("sd", -0.5)])
+def test_ragged_tiles_in_the_staged_launch(dtype, beta):
+    """Ragged tiles that the staged kernel moves in its own launch: one ragged dimension or two,
+    remainders of one element, of all but one and of whole vectors, limits on and off the vector grid,
+    misaligned pointers, claimed tiles, shifted runs, bulk copies and deep rings, bit for bit against the
+    oracle; and the same launch captured and replayed."""
+    seen = set()
+    for perm, size in [([1, 0], [65, 129]), ([1, 0], [127, 95]), ([1, 0, 2], [36, 68, 5]), ([1, 0], [100, 412]),
+                       ([2, 1, 0], [11, 2, 1093]), ([2, 0, 1], [67, 31, 53]), ([0, 2, 1], [3, 97, 61]),
+                       ([1, 2, 0], [26, 653, 8]), ([3, 1, 0, 2], [17, 3, 7, 29])]:
+        for tuning in ({"tile_elems": 512}, {"tile_elems": 1024, "round_robin": -1, "blocks": 5},
+                       {"tile_elems": 1024, "shifted_runs": 1}, {"tile_elems": 2048, "bulk_copies": 1, "stages": 6}):
+            for offset in (0, 1):
+                desc = check_case(perm, size, dtype, 1.5, beta, tuning=tuning, offset=offset)
+                t = desc.get("tile") or {}
+                seen.add((t.get("ragged_inline"), t.get("shifted_runs"), t.get("bulk")))
+    assert {k[0] for k in seen} >= {1, 2}, seen
+
+
 def test_claimed_tiles_with_concurrent_launches_and_slot_reuse():
     """The staged kernel's tiles claimed from the plan's counters: one plan launched on four streams
     at once (different counter slots), then 150 launches in a row on one stream (every slot used and

@@ -472,3 +472,50 @@ def test_lane_maps():
                 wa, wb = _oracle_pairs(perm, size, None, None)
                 assert dict(zip(bb.tolist(), a.tolist())) == dict(zip(wb.tolist(), wa.tolist()))
     assert maps >= 10 and sorted_runs >= 2, (maps, sorted_runs)
+
+
+def test_ragged_tiles_moved_by_vectors_have_whole_vectors():
+    """When the staged kernel moves ragged tiles by vectors (ragged_inline 1), every vector of a ragged
+    tile is valid as a whole or not at all, in A order (vecA) and in B order (vecB), and at aligned
+    offsets; by single elements (2) otherwise, and never when the schedule asks for the ragged kernel."""
+    rng = np.random.default_rng(31)
+    seen = {0: 0, 1: 0, 2: 0}
+    for it in range(400):
+        perm, size, lda, ldb = _random_problem(rng, max_rank=4, max_ext=70, pad=it % 3 == 0)
+        dtype = ["s", "d", "zc", "sd", "ds", "c"][it % 6]
+        tu = {"tile_elems": [128, 512, 2048][it % 3]}
+        if it % 4 == 3:
+            tu["shifted_runs"] = 1
+        try:
+            j = plan_host_json(perm, size, dtype, it % 2 == 1, lda, ldb, tu)
+            kind, b = kernel_sim.host_desc(perm, size, dtype, it % 2 == 1, lda, ldb, tu)
+        except TTCError:
+            continue
+        if kind != 1:
+            continue
+        t = kernel_sim.parse_tile(b)
+        if t["nrag0"] + t["nrag1"] == 0 or not t["async_ok"]:
+            assert j["tile"]["ragged_inline"] == 0
+            continue
+        mode = j["tile"]["ragged_inline"]
+        seen[mode] += 1
+        assert plan_host_json(perm, size, dtype, it % 2 == 1, lda, ldb, dict(tu, ragged=1))["tile"]["ragged_inline"] == 0
+        if mode != 1:
+            continue
+        assert not t["shiftA"]
+        P = t["P"]
+        for ts, V in (("tsA", j["vecA"]), ("tsB", j["vecB"])):
+            p = np.arange(P, dtype=np.int64)
+            ok = {}
+            for k, bd in enumerate(t["bd"]):
+                c = fdiv_mod(p, bd, ts)
+                g = next(g for g in t["g"] if g["blocked"] == k)
+                for lim in {g["e"], g["n"] - (g["div"][0] - 1) * g["e"]}:
+                    ok[k, lim] = c < lim
+                    assert (ok[k, lim].reshape(-1, V).all(1) == ok[k, lim].reshape(-1, V).any(1)).all(), (perm, size, tu)
+    assert seen[1] >= 40 and seen[2] >= 10, seen
+
+
+def fdiv_mod(p, bd, ts):
+    c = kernel_sim.fdiv(p, bd[ts]).astype(np.int64)
+    return c - kernel_sim.fdiv(c, bd["ext"]).astype(np.int64) * bd["ext"][0]

@@ -146,8 +146,8 @@ def schedule_alternatives(p: Problem, desc: dict, k: int) -> list[dict]:
 
 def staged_claims(p: Problem, tuning: dict, desc: dict) -> bool:
     """Whether the staged kernel claims tiles from counters under this schedule: asked for
-    (round_robin -1), or the planner's rule for round_robin 0 - tiles of 16 KiB or more (A, B and B
-    read back) with 16 or more per CTA (CTAs estimated as SMs x the schedule's CTAs per SM, else as
+    (round_robin -1), or the planner's rule for round_robin 0 - a call that moves 128 MB or more (150 MB
+    when B is read back) with 8 or more tiles per CTA (CTAs estimated as SMs x the schedule's CTAs per SM, else as
     many as the ring's shared memory lets share an SM)."""
     rr = tuning.get("round_robin", 0)
     if rr != 0:
@@ -156,14 +156,13 @@ def staged_claims(p: Problem, tuning: dict, desc: dict) -> bool:
     if desc.get("kernel") != "tile" or not t.get("P"):
         return False
     ta, tb = split_dtype(p.dtype)
-    tile_bytes = t["P"] * (ELEM_BYTES[ta] + ELEM_BYTES[tb] * (2 if p.beta_nonzero else 1))
     c = tuning.get("ctas_per_sm") or t.get("ctas_per_sm") or 0
     if not c:
         stage = t["P"] * ELEM_BYTES[ta] * 1.07 + (t["P"] * ELEM_BYTES[tb] if p.beta_nonzero else 0)
         S = tuning.get("stages") or t.get("stages") or 3
         c = max(1, min(4, int(227 * 1024 // (S * stage + 3 * 1024))))
     ctas = tuning.get("blocks") or c * SMS
-    return tile_bytes >= 16 * 1024 and t.get("ntiles", 0) >= 16 * ctas
+    return p.bytes() >= (150_000_000 if p.beta_nonzero else 128_000_000) and t.get("ntiles", 0) >= 8 * ctas
 
 
 def fused_groups(p: Problem):

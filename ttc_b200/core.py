@@ -171,10 +171,11 @@ def transpose(A, B, perm: Sequence[int], size: Optional[Sequence[int]] = None, a
 
 def describe_launches(d: dict) -> int:
     """Kernels a call of the plan described by `d` launches: its kernel, and for a staged tile plan
-    with ragged tiles either its edge plans' kernels or the element-wise ragged-tile kernel."""
+    whose kernel leaves ragged tiles to others either its edge plans' kernels or the element-wise
+    ragged-tile kernel."""
     t = d.get("tile") or {}
     n = 1
-    if t.get("async") and t.get("ragged_tiles", 0) > 0 and d.get("tile_variant", 0) in (0, 3):
+    if not t.get("ragged_inline") and t.get("async") and t.get("ragged_tiles", 0) > 0 and d.get("tile_variant", 0) in (0, 3):
         edges = d.get("edges") or []
         n += sum(describe_launches(e["plan"]) for e in edges) if edges else 1
     return n

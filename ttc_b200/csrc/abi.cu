@@ -90,8 +90,10 @@ using ttcb::needs_large_smem;
 // for it with round_robin = -1, or the planner's rule below); otherwise it takes the round-robin
 // order.
 static bool uses_claims(const ttcb_plan* p) { return p->claim_words != nullptr; }
-static constexpr int64_t kClaimMinTileBytes = 16 * 1024;
-static constexpr int kClaimMinTilesPerCta = 16;
+static constexpr int64_t kClaimMinBytes = 128 * 1000 * 1000, kClaimMinBytesBeta = 150 * 1000 * 1000;
+static constexpr int kClaimMinTilesPerCta = 8;
+static constexpr int64_t kClaimPairTileBytes = 13 * 1024;
+static constexpr int64_t kClaimSingleTileBytes = 20 * 1024;
 // The staged kernel moves A runs with bulk copies when the plan's layout allows it and A's pointer
 // meets the layout's alignment (shifted runs take any pointer; plain runs need the 16-byte vector).
 static bool uses_bulk(const ttcb_plan* p, const TileDesc* td, int va, int EA) {
@@ -164,20 +166,32 @@ static ttcb_status plan_finish_device(ttcb_plan* p) {
     }
     if (td->async_ok) {
       // Tiles are claimed in order from counters when the schedule asks for it, or by default for
-      // tiles of 16 KiB or more (A, B and B read back) when every CTA has at least 16 of them. Timed
-      // over the 200 MiB sweep back to back, claims made such tiles 2-15% faster (CTAs stay on
-      // neighbouring tiles, so the tiles in motion span a narrow stretch of A and B) and smaller
-      // ones up to 19% slower (the claim's round trip is not hidden behind a short tile); a CTA
-      // claims its first S tiles at once, which leaves CTAs idle when each has only a few (the 147 MB
-      // 1000x768x16 transposition, 11 tiles per CTA: 10% slower).
+      // calls that move 128 MB or more (150 MB when B is read too; the L2 holds 126 MB) with 8 tiles or
+      // more per CTA. Past L2, the
+      // CTAs' drift apart under the round-robin order spreads the tiles in motion over A and B: back to
+      // back over the 200 MiB sweep, claims against round robin took 0.78-0.97 of the time on 52 of the
+      // 61 tile plans and 1.00-1.06 on the others (tiles of 7-11 KiB), the sweep 6.24 against 6.62 ms; 156 MB
+      // (11 tiles of 48 KiB per CTA) 27.7 against 31.3 us. Within L2 the order does not matter and the claims
+      // cost (51 MB in tiles of 8 KiB: 15.5 against 12.2 us; 93 MB: 18.9 against 18.3; 147 MB with B read
+      // back, 98 MB of tensors: 27.0 against 26.5).
       const int EA = dtype_bytes(p->ta);
-      s = grid_for(staged_kernel_id(p, td, td->reg_ok, false), p->smem_async, &p->blocks_async, td->nfull);
+      const int64_t tiles = (int64_t)td->nfull + (p->rag_inline ? (int64_t)td->nrag0 + td->nrag1 : 0);
+      s = grid_for(staged_kernel_id(p, td, td->reg_ok, false), p->smem_async, &p->blocks_async, tiles);
       if (s != TTCB_OK) return s;
-      const int64_t tile_bytes = (int64_t)td->P * (EA + dtype_bytes(p->tb) * (p->beta_nonzero ? 2 : 1));
-      const bool claims_by_default = p->tuning.round_robin == 0 && tile_bytes >= kClaimMinTileBytes &&
+      const int64_t elem_bytes = EA + dtype_bytes(p->tb) * (p->beta_nonzero ? 2 : 1);
+      const bool claims_by_default = p->tuning.round_robin == 0 && p->N * elem_bytes >= (p->beta_nonzero ? kClaimMinBytesBeta : kClaimMinBytes) &&
                                      td->nfull >= (int64_t)kClaimMinTilesPerCta * p->blocks_async;
-      // two tiles per claim: back to back over the sweep, 0.3% faster than one (three: 0.3% slower)
-      p->claim_group = p->tuning.claim_group > 0 ? std::min(p->tuning.claim_group, 64) : 2;
+      // Tiles per claim: four of tiles under 13 KiB, whose claim would not be back in time (back to back
+      // over the sweep, four against two: 0.88-0.99 of the time for tiles of 6-12 KiB, 1.01-1.08 for tiles
+      // of 14 KiB and more), else two; but one of tiles of 20 KiB and more in a three-stage ring whose B
+      // runs are at most 160 bytes, so that neighbours, which share lines or DRAM bursts of B, are
+      // written by different CTAs at the same time (one against two on 8 such shapes of 200 MiB: 0.88-0.99
+      // of the time; with longer runs or deeper rings 1.00-1.17).
+      const int64_t tile_bytes = td->P * elem_bytes;
+      const bool short_b = tile_bytes >= kClaimSingleTileBytes && td->nstages == 3 &&
+                           td->LB * (int64_t)dtype_bytes(p->tb) <= 160;
+      const int group = tile_bytes < kClaimPairTileBytes ? 4 : short_b ? 1 : 2;
+      p->claim_group = p->tuning.claim_group > 0 ? std::min(p->tuning.claim_group, ttcb::kDecodeBatch) : group;
       if (p->tuning.round_robin == -1 || claims_by_default) {
         e = cudaMalloc(&p->claim_words, sizeof(unsigned int) * 2 * ttcb::kClaimSlots);
         if (e != cudaSuccess) {
@@ -201,9 +215,9 @@ static ttcb_status plan_finish_device(ttcb_plan* p) {
           return cuda_fail(e, "cudaMemset of the wait status");
       }
       s = grid_for(staged_kernel_id(p, td, td->reg_ok, uses_bulk(p, td, p->vecA, EA)), p->smem_async, &p->blocks_async,
-                   td->nfull);
+                   tiles);
       if (s != TTCB_OK) return s;
-      if (td->nrag0 + td->nrag1 > 0) {
+      if (td->nrag0 + td->nrag1 > 0 && !p->rag_inline) {
         s = grid_for(TTCB_KERNEL_TILE_RAGGED, p->smem_ragged, &p->blocks_ragged, (int64_t)td->nrag0 + td->nrag1);
         if (s != TTCB_OK) return s;
         if (p->depth > 0) return TTCB_OK;  // an edge plan runs on its parent's side stream
@@ -226,7 +240,8 @@ static ttcb_status plan_finish_device(ttcb_plan* p) {
   return TTCB_OK;
 }
 
-// Launches a checked plan on stream st. The staged kernel moves complete tiles only; a plan with
+// Launches a checked plan on stream st. The staged kernel moves the complete tiles and, where that is
+// the cheaper way (plan_rag_inline), the ragged ones. Any other plan with
 // ragged tiles forks its side stream from st before the staged kernel and joins it back after, and
 // the side stream moves the ragged tiles beside the staged kernel (they write disjoint parts of B):
 // through the edge plans when there are some, else with the element-wise ragged-tile kernel. An
@@ -264,7 +279,7 @@ static ttcb_status launch_plan(const ttcb_plan* p, const void* A, void* B, const
   if (needs_large_smem(smem)) allow_large_smem(k.func);
   const TileDesc* td = reinterpret_cast<const TileDesc*>(p->host_desc.data());
   const bool ragged = ttcb_is_staged_kernel(kernel) && td->nrag0 + td->nrag1 > 0;
-  if (!ragged) {
+  if (!ragged || p->rag_inline) {
     e = k.fn(p, A, B, alpha, beta, st, blocks);
     if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
     return TTCB_OK;

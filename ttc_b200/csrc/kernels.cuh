@@ -549,18 +549,164 @@ __host__ __device__ inline size_t async_smem_bytes(int S, int stage_elems, int P
 // tile decode per iteration instead of a whole one.
 struct TileInfo {
   int64_t bA, bB;
-  int32_t state;  // 1: complete tile, 0: ragged tile, -1: past the last tile
+  int32_t state;  // 1: complete tile, 0: ragged tile (limits lim0, lim1), -1: past the last tile
   int32_t lim0, lim1, pad_;
 };
 
 // Static shared memory of the staged kernel (descriptor header + tile ring), on top of its dynamic
 // shared memory.
-constexpr int kDecodeBatch = 8;              // staged kernel: tiles decoded per batch
+constexpr int kDecodeBatch = 8;              // staged kernel: tiles decoded per batch (and at most per claim)
 constexpr int kInfoRing = 2 * kDecodeBatch;  // decoded-tile ring entries (tile j in entry j % kInfoRing)
 constexpr int kMaxStages = 7;                // S - 2 = D tiles in flight, D < kDecodeBatch
+static_assert(kMaxStages - 2 + kDecodeBatch + 2 <= kInfoRing, "claimed tiles must replace finished ones only");
 static_assert(kMaxStages - 2 < kDecodeBatch && kMaxStages - 2 <= 5,
               "tiles in flight must be decoded a batch ahead and covered by the copy-group wait");
 constexpr size_t kAsyncStaticSmem = sizeof(TileDesc) + kInfoRing * sizeof(TileInfo) + kMaxStages * sizeof(uint64_t);
+
+// Tile index of the r-th ragged tile (see TileDesc::rag_a): mixed radix over the grid dimensions
+// with the ragged dimension pinned to its last block (and, in the second part, rag_a below its last).
+__device__ __forceinline__ uint32_t ragged_tile_index(const TileDesc& d, uint32_t r) {
+  int fixed = d.rag_a, excl = -1;
+  if (r >= (uint32_t)d.nrag0) {
+    r -= (uint32_t)d.nrag0;
+    fixed = d.rag_b;
+    excl = d.rag_a;
+  }
+  uint32_t t = 0, M = 1;
+  for (int k = 0; k < d.ngrid; ++k) {
+    const uint32_t cnt = d.g[k].div.d;
+    uint32_t c;
+    if (k == fixed) {
+      c = cnt - 1;
+    } else {
+      const uint32_t radix = (k == excl) ? cnt - 1 : cnt;
+      c = r % radix;
+      r /= radix;
+    }
+    t += c * M;
+    M *= cnt;
+  }
+  return t;
+}
+
+// Ragged tiles inside the staged kernel (kernel argument `rag`): CTA b moves ragged tiles b, b + G, ..
+// before its complete tiles, through two stages of its ring. A launch of its own for them costs a fork
+// to a side stream and a join back: about 4 us on the device, where the call after it can then not
+// start while this one drains, and 5.5 us on the host. Elements go V at a time when every tile limit falls
+// on a multiple of V in both orders (kRagVec: V is the access width), else one at a time. The pass is
+// a call of its own, ahead of the ring's set-up, so that the ring keeps its registers (with the ragged
+// tiles in the ring's own order, scalar fp32 instantiations spilled and ran 4-9% slower).
+enum { kRagNone = 0, kRagVec = 1, kRagScalar = 2 };
+
+// Whether A-order (B-order: tsB) position p lies within the tile's limits.
+template <bool ORDER_B>
+__device__ __forceinline__ bool ragged_in(const TileDesc& d, uint32_t p, int lim0, int lim1) {
+  bool ok = true;
+  for (int b = 0; b < d.nblocked; ++b) {
+    const uint32_t c = fdiv(p, ORDER_B ? d.bd[b].tsB : d.bd[b].tsA);
+    const uint32_t cc = c - fdiv(c, d.bd[b].ext) * d.bd[b].ext.d;
+    ok = ok && (int)cc < (b == 0 ? lim0 : lim1);
+  }
+  return ok;
+}
+
+// The CTA's ragged tiles (see kRagVec), V = VA (VB) elements at a time, in two of the S stages at `smem`
+// (sbytes each; the B tile a_bytes in). The tables go to shared memory (run tables behind the stages,
+// the gather table in the third stage) and the first tile is decoded before the previous launch is
+// waited for: a small call's time is the latency of its one ragged tile, and with the tables read from
+// global memory after the wait 46 tiles of fp64 took 6.2 us. Two entries of info are used. Ends
+// with every thread done with the stages.
+template <typename TA, typename TB, int VA, int VB, bool BETA, bool STREAM>
+__device__ __noinline__ void ragged_pass(const TileDesc& d, const unsigned char* desc, const TA* __restrict__ A,
+                                         TB* __restrict__ B, TA alpha, TB beta, unsigned char* smem, uint32_t a_bytes,
+                                         uint32_t sbytes, TileInfo* info, int a0) {
+  constexpr int VM = 16 / (int)sizeof(TA);
+  const int P = d.P, LA = d.LA, LB = d.LB, nsegA = d.nsegA, nsegB = d.nsegB;
+  const uint32_t R = (uint32_t)(d.nrag0 + d.nrag1), G = gridDim.x;
+  int64_t* segA = reinterpret_cast<int64_t*>(smem + d.nstages * sbytes);
+  int64_t* segB = segA + nsegA;
+  uint16_t* gtab = reinterpret_cast<uint16_t*>(smem + 2 * sbytes);
+  auto decode = [&](uint32_t r, TileInfo& ti) {
+    int lim[2];
+    decode_tile(d, ragged_tile_index(d, r), ti.bA, ti.bB, lim);
+    ti.lim0 = lim[0];
+    ti.lim1 = lim[1];
+  };
+  auto shift_of = [&](const TileInfo& ti) { return d.shiftA ? (int)((a0 + ti.bA) & (int64_t)(VM - 1)) : 0; };
+  auto issue = [&](const TileInfo& ti, uint32_t stage) {
+    const uint32_t sb = smem_u32(smem) + stage * sbytes;
+    const TA* At = A + ti.bA;
+    const int x = shift_of(ti), lim0 = ti.lim0, lim1 = ti.lim1;
+    for (int p = (int)threadIdx.x * VA; p < P; p += kThreads * VA) {
+      if (!ragged_in<false>(d, (uint32_t)p, lim0, lim1)) continue;
+      const int s = (int)fdiv((uint32_t)p, d.divLA);
+      const int64_t seg = segA[s];
+      const int at = d.shiftA ? s * d.shiftW + (int)(seg & (int64_t)(VM - 1)) + x + (p - s * LA)
+                              : p + (int)fdiv((uint32_t)p, d.divSigmaA) * d.padA;
+      cp_async<VA * sizeof(TA)>(sb + (uint32_t)at * (uint32_t)sizeof(TA), At + (seg + (p - s * LA)));
+    }
+    if (BETA) {
+      const TB* Bt = B + ti.bB;
+      for (int q = (int)threadIdx.x * VB; q < P; q += kThreads * VB) {
+        if (!ragged_in<true>(d, (uint32_t)q, lim0, lim1)) continue;
+        const int s = (int)fdiv((uint32_t)q, d.divLB);
+        cp_async<VB * sizeof(TB)>(sb + a_bytes + (uint32_t)(q * sizeof(TB)), Bt + (segB[s] + (q - s * LB)));
+      }
+    }
+    cp_async_commit();
+  };
+  {
+    const int64_t* gA = reinterpret_cast<const int64_t*>(desc + d.off_segA);
+    const int64_t* gB = reinterpret_cast<const int64_t*>(desc + d.off_segB);
+    const uint32_t* gG = reinterpret_cast<const uint32_t*>(desc + d.off_gtab);
+    for (int i = threadIdx.x; i < nsegA; i += kThreads) segA[i] = gA[i];
+    for (int i = threadIdx.x; i < nsegB; i += kThreads) segB[i] = gB[i];
+    for (int i = threadIdx.x; i < (P + 1) / 2; i += kThreads) reinterpret_cast<uint32_t*>(gtab)[i] = gG[i];
+  }
+  uint32_t r = blockIdx.x;
+  if (threadIdx.x == 0) decode(r, info[0]);
+  __syncthreads();
+  pdl_wait_previous();
+  issue(info[0], 0);
+  for (uint32_t cur = 0;; cur ^= 1) {
+    const uint32_t rn = r + G;
+    const bool more = rn < R;
+    if (more) {
+      if (threadIdx.x == 0) decode(rn, info[cur ^ 1]);
+      __syncthreads();  // also: every thread is done with the other stage
+      issue(info[cur ^ 1], cur ^ 1);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+    const TileInfo& ti = info[cur];
+    const TA* st = reinterpret_cast<const TA*>(smem + cur * sbytes) + shift_of(ti);
+    const TB* sB = reinterpret_cast<const TB*>(smem + cur * sbytes + a_bytes);
+    TB* Bt = B + ti.bB;
+    const int lim0 = ti.lim0, lim1 = ti.lim1;
+    for (int q = (int)threadIdx.x * VB; q < P; q += kThreads * VB) {
+      if (!ragged_in<true>(d, (uint32_t)q, lim0, lim1)) continue;
+      const int s = (int)fdiv((uint32_t)q, d.divLB);
+      Vec<TB, VB> out;
+#pragma unroll
+      for (int j = 0; j < VB; ++j) {
+        const TA t = scale_a(alpha, st[gtab[q + j]]);
+        if (BETA)
+          out.v[j] = combine<TA, TB>(t, sB[q + j], beta);
+        else
+          out.v[j] = finish<TA, TB>(t);
+      }
+      st_vec<TB, VB>(Bt + (segB[s] + (q - s * LB)), out, STREAM);
+    }
+    if (!more) break;
+    r = rn;
+    __syncthreads();
+  }
+  // a bulk copy may follow these generic-proxy writes into a stage
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  __syncthreads();
+}
 
 // REG: every tile-relative offset of this thread lives in registers (tiles of at most kRegVec
 // vectors per thread and side whose offsets fit 32 bits and whose staged bytes fit 16 bits): A
@@ -569,13 +715,14 @@ constexpr size_t kAsyncStaticSmem = sizeof(TileDesc) + kInfoRing * sizeof(TileIn
 // per vector from the run tables in shared memory, with the gather positions in registers while
 // P <= kRegPos * kThreads and in shared memory beyond. The number of stages (3 to kMaxStages) is the
 // descriptor's.
-// DYN: tiles are claimed in order from a counter in global memory (sched[0]) as the CTA goes, instead
-// of the fixed round-robin blockIdx.x + k * gridDim.x. CTAs then stay on neighbouring tiles however
-// their speeds differ, so the tiles in motion stay within a narrow span of A and B, and the last
-// tiles go to whichever CTAs are free. Each claim takes claim_group consecutive tiles and is issued
-// a group before its tiles are used; the last CTA to finish (sched[1] counts them) sets both words back to zero for the next
-// launch that uses them, which runs after this grid completes (stream order, and griddepcontrol.wait
-// before the first claim when the launch overlaps its predecessor).
+// DYN: after the first D + 2 tiles of each CTA (round robin), tiles are claimed in order from a counter
+// in global memory (sched[0]) as the CTA goes, instead of the fixed round-robin first + k * gridDim.x.
+// CTAs then stay on neighbouring tiles however their speeds differ, so the tiles in motion stay within
+// a narrow span of A and B, and the last tiles go to whichever CTAs are free. Each claim takes
+// claim_group (1..8) consecutive tiles, decoded by as many lanes at once. The last CTA to finish
+// (sched[1] counts them) sets both words back to zero for the next launch that uses them, which runs
+// after this grid completes (stream order, and griddepcontrol.wait before the first claim when the
+// launch overlaps its predecessor). A launch of at most (D + 2) * gridDim.x tiles claims none.
 // a0 (shifted A runs only): A's pointer is a0 elements past a 16-byte boundary.
 // BULK (descriptor's bulkA; VA is the 16-byte vector): the lanes of warp 0 move each A run of a
 // tile with one bulk copy, and the stage's mbarrier counts the bytes; every thread waits on it before
@@ -586,7 +733,8 @@ template <typename TA, typename TB, int VA, int VB, bool BETA, bool STREAM, bool
 __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB * sizeof(TB), BETA))
     tile_async_kernel(
     const TileDesc* __restrict__ desc, const TA* __restrict__ A, TB* __restrict__ B, TA alpha, TB beta,
-    unsigned int* __restrict__ sched, int a0, unsigned int* __restrict__ wait_status, unsigned int claim_group) {
+    unsigned int* __restrict__ sched, int a0, unsigned int* __restrict__ wait_status, unsigned int claim_group,
+    int rag) {
   static_assert(!BULK || VA * sizeof(TA) == 16, "bulk copies move runs of whole 16-byte vectors");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ TileDesc d;  // the descriptor header, read once per CTA
@@ -607,6 +755,13 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
   const bool reg_pos = REG || P <= kRegPos * kThreads;
   const unsigned char* base = reinterpret_cast<const unsigned char*>(desc);
   const uint16_t* ggtab = reinterpret_cast<const uint16_t*>(base + d.off_gtab);
+  const uint32_t nrag = rag ? (uint32_t)(d.nrag0 + d.nrag1) : 0u;
+  if (blockIdx.x < nrag) {
+    if (rag == kRagVec)
+      ragged_pass<TA, TB, VA, VB, BETA, STREAM>(d, base, A, B, alpha, beta, smem_raw, a_bytes, sbytes, info, a0);
+    else
+      ragged_pass<TA, TB, 1, 1, BETA, STREAM>(d, base, A, B, alpha, beta, smem_raw, a_bytes, sbytes, info, a0);
+  }
   {
     const int64_t* gA = reinterpret_cast<const int64_t*>(base + d.off_segA);
     const int64_t* gB = reinterpret_cast<const int64_t*>(base + d.off_segB);
@@ -712,8 +867,10 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
     return 0u;
   };
 
-  const uint32_t ntiles = (uint32_t)d.nfull;  // the ragged tiles are the ragged-tile kernel's
+  const uint32_t ntiles = (uint32_t)d.nfull;
   const uint32_t G = gridDim.x;
+  // the fixed order starts after the CTAs that had a ragged tile (which take their first complete tile last)
+  const uint32_t first = nrag ? (blockIdx.x + G - nrag % G) % G : blockIdx.x;
   const uint32_t stage0 = smem_u32(smem_raw);
 
   auto decode_into = [&](uint32_t t, TileInfo& ti) {
@@ -729,7 +886,7 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
   auto shift_of = [&](const TileInfo& ti) -> int { return shift ? (int)((a0 + ti.bA) & (VA - 1)) : 0; };
 
   auto issue = [&](const TileInfo& ti, int stage) {
-    if (ti.state != 1) return;  // ragged tiles are moved by the ragged-tile kernel
+    if (ti.state != 1) return;
     const int x = shift_of(ti);
     const TA* At = A + (ti.bA - x);  // 16-byte aligned with shifted runs
     const TB* Bt = B + ti.bB;
@@ -857,9 +1014,12 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
   // (k - 2) every thread finished writing out before the barrier of iteration k - 1. Tiles are
   // decoded in batches (see TileInfo).
   const int D = S - 2;
-  // DYN: thread 0 claims claim_group consecutive tiles per atomic, one group ahead: `pending` is the
-  // first tile of the next group, `cbase` of the current one, `cleft` the current group's tiles left
-  unsigned int pending = 0, cbase = 0, cleft = 0;
+  // DYN: tiles 0 .. (D + 2) * G - 1 go round robin (decoded before the previous launch is waited for);
+  // then warp 0 takes claim_group consecutive tiles per claim, issued a group ahead. Lane 0's `pending`
+  // is the first tile of the next group; `cleft` counts the iterations until it is decoded.
+  unsigned int pending = ntiles, cleft = 0;
+  const unsigned int claim0 = (unsigned int)(D + 2) * G;
+  const bool claiming = DYN && claim0 < ntiles;
   uint32_t phase = 0;        // BULK: bit s = parity of the next phase of stage s's barrier
   if constexpr (BULK) {
     if (tid == 0) {
@@ -868,23 +1028,15 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
     }
   }
   if constexpr (DYN) {
-    // claims touch no tensor data, but the previous launch's reset of the counter must be visible
-    pdl_wait_previous();
-    if (tid < 32) {
-      unsigned int base = 0;
-      if (tid == 0) {
-        base = atomicAdd(&sched[0], (unsigned int)(D + 2));
-        pending = atomicAdd(&sched[0], claim_group);
-      }
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (tid < D + 2) decode_into(base + tid, info[tid]);
-    }
+    if (tid < D + 2) decode_into(claiming ? first * (D + 2) + tid : first + tid * G, info[tid]);
   } else {
-    if (tid < kInfoRing) decode_into(blockIdx.x + tid * G, info[tid]);
+    if (tid < kInfoRing) decode_into(first + tid * G, info[tid]);
   }
   __syncthreads();
   // everything above reads the plan's descriptor only; A and B are touched from here on
   pdl_wait_previous();
+  // (the previous launch's reset of the counter is visible from here)
+  if (claiming && tid == 0) pending = claim0 + atomicAdd(&sched[0], claim_group);
   for (int j = 0; j < D; ++j) {
     issue(info[j], j);
     cp_async_commit();
@@ -895,7 +1047,7 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
     if constexpr (DYN) {
       if (info[k % kInfoRing].state < 0) break;  // claims grow, so every later one is past the end too
     } else {
-      const uint32_t t = blockIdx.x + k * G;
+      const uint32_t t = first + k * G;
       if (t >= ntiles) break;
     }
     issue(info[(k + D) % kInfoRing], nxt);
@@ -931,20 +1083,20 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
       __syncthreads();
     }
     if constexpr (DYN) {
-      // the tile of iteration k + D + 2 (read after the next barrier), and the next claim, whose
-      // result thread 0 needs only an iteration later (decoding here, before thread 0's own stores,
-      // timed 3% faster over the 200 MiB sweep than after them)
-      if (tid == 0) {
-        if (cleft == 0) {
-          cbase = pending;
-          cleft = claim_group;
-          pending = atomicAdd(&sched[0], claim_group);
+      // the tiles of iterations k + D + 2 .. k + D + 1 + claim_group, one lane each (the first is read
+      // after the next barrier; the ring entries they replace are of tiles before k), and the next
+      // claim, whose result is needed a group later
+      if (cleft == 0) {
+        cleft = claim_group;
+        if (tid < 32) {
+          const unsigned int t = __shfl_sync(0xffffffffu, pending, 0) + (unsigned int)tid;
+          if (tid < (int)claim_group) decode_into(t, info[(k + D + 2 + tid) % kInfoRing]);
+          if (claiming && tid == 0) pending = claim0 + atomicAdd(&sched[0], claim_group);
         }
-        decode_into(cbase + (claim_group - cleft), info[(k + D + 2) % kInfoRing]);
-        --cleft;
       }
+      --cleft;
     } else {
-      const uint32_t t = blockIdx.x + k * G;
+      const uint32_t t = first + k * G;
       if (tid < kDecodeBatch && k % kDecodeBatch == 0 && k != 0)
         decode_into(t + (kDecodeBatch + tid) * G, info[(k + kDecodeBatch + tid) % kInfoRing]);
     }
@@ -1002,7 +1154,7 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
   cp_async_wait<0>();
   if constexpr (DYN) {
     // every claim of this CTA is done; the last CTA to get here resets the counter words
-    if (tid == 0) {
+    if (claiming && tid == 0) {
       __threadfence();
       if (atomicAdd(&sched[1], 1u) == gridDim.x - 1) {
         atomicExch(&sched[0], 0u);
@@ -1076,32 +1228,6 @@ __device__ __forceinline__ void ragged_store(const TileDesc& d, const RaggedTabl
 // Shared memory: two tile buffers of `slots` bytes each, then the per-element tables.
 __host__ __device__ inline size_t ragged_smem_bytes(int phys_size, int elem_bytes, int P) {
   return 2 * tile_slots_bytes(phys_size, elem_bytes) + 16 * (size_t)P + al16((size_t)2 * P);
-}
-
-// Tile index of the r-th ragged tile (see TileDesc::rag_a): mixed radix over the grid dimensions
-// with the ragged dimension pinned to its last block (and, in the second part, rag_a below its last).
-__device__ __forceinline__ uint32_t ragged_tile_index(const TileDesc& d, uint32_t r) {
-  int fixed = d.rag_a, excl = -1;
-  if (r >= (uint32_t)d.nrag0) {
-    r -= (uint32_t)d.nrag0;
-    fixed = d.rag_b;
-    excl = d.rag_a;
-  }
-  uint32_t t = 0, M = 1;
-  for (int k = 0; k < d.ngrid; ++k) {
-    const uint32_t cnt = d.g[k].div.d;
-    uint32_t c;
-    if (k == fixed) {
-      c = cnt - 1;
-    } else {
-      const uint32_t radix = (k == excl) ? cnt - 1 : cnt;
-      c = r % radix;
-      r /= radix;
-    }
-    t += c * M;
-    M *= cnt;
-  }
-  return t;
 }
 
 template <typename TA, typename TB, bool BETA, bool STREAM>

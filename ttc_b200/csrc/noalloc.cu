@@ -139,12 +139,13 @@ extern "C" ttcb_status ttcb_transpose_noalloc(int rank, const int* perm, const i
       cudaSuccess)
     return na_cuda(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
   if (per_sm < 1) return na_fail(TTCB_ERR_UNSUPPORTED, "tile does not fit in shared memory");
-  const int64_t work = td->nfull, resident = (int64_t)per_sm * sms;
+  const int64_t nrag = (int64_t)td->nrag0 + td->nrag1;
+  const int64_t work = td->nfull + (p.rag_inline ? nrag : 0), resident = (int64_t)per_sm * sms;
   const int64_t per = (work + resident - 1) / resident;
   p.blocks_async = (int)std::max<int64_t>((work + per - 1) / per, 1);
   e = k.fn(&p, A, B, alpha, beta, st, p.blocks_async);
-  if (e == cudaSuccess && td->nrag0 + td->nrag1 > 0) {
-    // the staged kernel moves complete tiles only; the ragged ones follow on the same stream
+  if (e == cudaSuccess && nrag > 0 && !p.rag_inline) {
+    // ragged tiles that the staged kernel leaves follow on the same stream
     ttcb::KernelRef kr = ttcb::pick_kernel(p.ta, p.tb, TTCB_KERNEL_TILE_RAGGED, 1, 1, variant);
     if (!kr.fn) {
       p.dev_desc = nullptr;
@@ -153,7 +154,7 @@ extern "C" ttcb_status ttcb_transpose_noalloc(int rank, const int* perm, const i
     if (ttcb::needs_large_smem(p.smem_ragged)) ttcb::allow_large_smem(kr.func);
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kr.func, ttcb::kThreads, p.smem_ragged)) ==
         cudaSuccess) {
-      const int64_t rw = (int64_t)td->nrag0 + td->nrag1, rres = (int64_t)std::max(per_sm, 1) * sms;
+      const int64_t rw = nrag, rres = (int64_t)std::max(per_sm, 1) * sms;
       const int64_t rper = (rw + rres - 1) / rres;
       e = kr.fn(&p, A, B, alpha, beta, st, (int)std::max<int64_t>((rw + rper - 1) / rper, 1));
     }

@@ -457,7 +457,9 @@ static constexpr double kTargetInFlightBytes = 18.0 * 1024 * 1024;
 // three and 12% with two, although single cases repeated alone ran faster with them) and picks the
 // S in 3..6 whose W comes nearest 18 MiB, among the rings that let two CTAs share an SM when there
 // are any: with S fixed at 3 or 4 for every case the sweep measured within 0.5% of the W rule, and for
-// single cases rings far from it lost 5-15%. Problems too small to
+// single cases rings far from it lost 5-15%. With beta != 0
+// three stages become four where two CTAs of those fit, but not three (tiles of 28-41 KiB): under claims
+// of two tiles 0.81-1.00 of the time of three stages on 13 shapes of 200 MiB. Problems too small to
 // fill the GPU twice keep the earlier rule (four stages while four CTAs fit, else three).
 // smem_for(S) is the dynamic shared memory of an S-stage ring; fixed_S (3..kMaxStages, else 0) is a
 // schedule's explicit ring depth.
@@ -495,6 +497,11 @@ static StageChoice choose_stages(int64_t P, int EA, int EB, bool beta, int vecA,
       bc = cmax;
     }
   }
+  auto ctas = [&](int S) {
+    return smem_for(S) > 200 * 1024 ? 0
+                                    : (int)((227 * 1024) / (smem_for(S) + (int64_t)ttcb::kAsyncStaticSmem + 1024));
+  };
+  if (beta && bS == 3 && !fixed && ctas(4) == 2) bS = 4;
   if (bS && nfull >= 2LL * 4 * kPlanSMs) out.S = bS;
   if (fixed) out.S = fixed_S;
   return out;
@@ -996,6 +1003,39 @@ bool unpack_raster(const ttcb_tuning& tu, int rank, int* order) {
   return true;
 }
 
+// Bytes of tile slots (complete-tile equivalents) that the ragged tiles may occupy beyond their own
+// elements when the staged kernel moves them: about 4 us at 6 TB/s, what the fork to the edge plans'
+// side stream and the join back cost on the device.
+static constexpr double kRagInlineWasteBytes = 24e6;
+// Time of a ragged tile against a complete one, by vectors and by single elements.
+static constexpr double kRagVecFactor = 1.3, kRagScalarFactor = 4.0;
+
+// How the staged kernel moves a tile plan's ragged tiles in its own launch (kRagVec / kRagScalar), or 0
+// when they are better moved by other launches or the schedule asks for those.
+static int plan_rag_inline(const ttcb_plan* p) {
+  if (p->kernel != TTCB_KERNEL_TILE || p->host_desc.empty() || p->tuning.ragged == 1) return 0;
+  const TileDesc* t = reinterpret_cast<const TileDesc*>(p->host_desc.data());
+  const int64_t nrag = (int64_t)t->nrag0 + t->nrag1;
+  if (!t->async_ok || nrag == 0 || (int64_t)t->nfull + nrag >= (int64_t(1) << 31)) return 0;
+  // vectors: within a vector of V consecutive positions all elements are valid or none is, when the
+  // dimension's stride in the numbering is a multiple of V, or its period and its limit are
+  bool vec = !t->shiftA;
+  double slots = 0;  // elements of the ragged tiles
+  for (int k = 0; k < t->ngrid; ++k) {
+    const GridDimDesc& g = t->g[k];
+    if (g.blocked < 0 || g.n % g.e == 0) continue;
+    const int64_t r = g.n % g.e, sa = t->bd[g.blocked].tsA.d, sb = t->bd[g.blocked].tsB.d;
+    if (sa % p->vecA != 0 && ((sa * r) % p->vecA != 0 || (sa * g.e) % p->vecA != 0)) vec = false;
+    if (sb % p->vecB != 0 && ((sb * r) % p->vecB != 0 || (sb * g.e) % p->vecB != 0)) vec = false;
+  }
+  slots = (double)nrag * t->P;
+  const double valid = (double)p->N - (double)t->nfull * t->P;
+  const double per = dtype_bytes(p->ta) + dtype_bytes(p->tb) * (p->beta_nonzero ? 2.0 : 1.0);
+  const double waste = (slots * (vec ? kRagVecFactor : kRagScalarFactor) - valid) * per;
+  if (waste > kRagInlineWasteBytes) return 0;
+  return vec ? ttcb::kRagVec : ttcb::kRagScalar;
+}
+
 // ------------------------------------------------------------------------------------------------
 ttcb_status plan_build_host(ttcb_plan* p, std::string& err) {
   const int r = p->rank;
@@ -1189,6 +1229,7 @@ ttcb_status plan_build_host(ttcb_plan* p, std::string& err) {
       build_tile_desc(p, best, EA);
     }
   }
+  p->rag_inline = plan_rag_inline(p);
   return TTCB_OK;
 }
 
@@ -1273,7 +1314,7 @@ std::string plan_describe_json(const ttcb_plan* p) {
       << ",\"reg\":" << t->reg_ok << ",\"smem_async\":" << p->smem_async
       << ",\"blocks_async\":" << p->blocks_async << ",\"ctas_per_sm\":" << p->ctas_per_sm
       << ",\"shifted_runs\":" << t->shiftA << ",\"bulk\":" << t->bulkA << ",\"lane_map\":" << (t->map_log2s >= 0 ? (1 << t->map_log2s) : 0) << ",\"claims\":" << (p->claim_words ? 1 : 0) << ",\"claim_group\":" << p->claim_group
-      << ",\"ragged_tiles\":" << (t->nrag0 + t->nrag1) << ",\"ext\":[";
+      << ",\"ragged_tiles\":" << (t->nrag0 + t->nrag1) << ",\"ragged_inline\":" << p->rag_inline << ",\"ext\":[";
     for (int d = 0; d < p->f.rank; ++d) o << (d ? "," : "") << p->tile_ext[d];
     o << "]}";
   } else if (p->kernel == TTCB_KERNEL_TILE && p->shape_only) {

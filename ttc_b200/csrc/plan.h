@@ -83,6 +83,10 @@ struct ttcb_plan {
   int smem_ragged = 0;    // its dynamic shared memory (two tile buffers + tables)
   int device = 0;
 
+  // staged kernel: how it moves the plan's ragged tiles itself (kRagVec or kRagScalar), or 0 when other
+  // launches do (edge plans, the ragged-tile kernel)
+  int rag_inline = 0;
+
   // ragged tiles: the fused dimensions whose last tile block is ragged and where that block starts
   int rag_dim[2] = {-1, -1};
   int64_t rag_start[2] = {0, 0};
