@@ -36,6 +36,26 @@ ttcb_status ttcb_mlp_adam(float* param, const float* grad, float* m, float* v, i
 ttcb_status ttcb_mlp_adam_l2(float* param, const float* grad, float* m, float* v, int n, float lr, float beta1,
                              float beta2, float eps, float weight_decay, int t, ttcb_stream_t stream);
 
+/* The same step on `count` parameter tensors (host arrays of device pointers and sizes) in one launch. */
+ttcb_status ttcb_mlp_adam_multi(int count, float* const* param, const float* const* grad, float* const* m,
+                                float* const* v, const int* n, float lr, float beta1, float beta2, float eps,
+                                float weight_decay, int t, ttcb_stream_t stream);
+
+/* The whole network (nin -> 128 -> 128 -> 1, ReLU between the layers) in one launch. params: host array of the
+ * six device tensors W1 [nin x 128], b1, W2 [128 x 128], b2, W3 [128], b3 [1]. X is rows x nin; H1 and H2
+ * [rows x 128] receive the hidden layers' outputs, out [rows] the network's. At most
+ * ttcb_mlp_passes_max_features() features. */
+ttcb_status ttcb_mlp_forward(int rows, int nin, const float* X, const float* const* params, float* H1, float* H2,
+                             float* out, ttcb_stream_t stream);
+
+/* Its gradients, given dout [rows] = d loss / d out: grads holds W1, b1, W2, b2, W3 and b3's one after the other.
+ * workspace: ttcb_mlp_backward_workspace(rows, nin) bytes of device memory, free again after the call (in
+ * stream order). */
+ttcb_status ttcb_mlp_backward(int rows, int nin, const float* X, const float* const* params, const float* H1,
+                              const float* H2, const float* dout, float* grads, void* workspace, ttcb_stream_t stream);
+size_t ttcb_mlp_backward_workspace(int rows, int nin);
+int ttcb_mlp_passes_max_features(void);
+
 #ifdef __cplusplus
 }
 #endif

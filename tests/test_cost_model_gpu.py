@@ -50,6 +50,44 @@ def test_gradients_match_cpu_oracle():
         assert rel <= 1e-4, rel
 
 
+@pytest.mark.parametrize("rows,nin", [(1, 1), (15, 3), (16, 4), (17, 96), (64, 127), (65, 128), (130, 129), (2048, 96),
+                                      (4096, 192), (4100, 61), (200, 193)])
+def test_whole_network_passes_at_block_edges(rows, nin):
+    """The forward pass against float64, and every gradient against float64 on the hidden layers' fp32
+    outputs (so that no unit's sign differs), at the edges of the row blocks (16 rows, 64 per cluster,
+    4096 per launch), of the feature pieces (128) and of what fits one launch (192; 193 goes layer by
+    layer): relative error in norm at most 1e-5 (sums of up to 4100 fp32 terms: 2^-24 times a few tens),
+    and the same bits twice."""
+    import torch
+    net = _net(nin, 128, rows)
+    rng = np.random.default_rng(nin)
+    X = torch.from_numpy(rng.standard_normal((rows, nin)).astype(np.float32)).cuda()
+    y = torch.from_numpy(rng.standard_normal((rows, 1)).astype(np.float32)).cuda()
+    for p in net.params[1::2]:
+        p.copy_(torch.from_numpy(rng.standard_normal(p.numel()).astype(np.float32)))
+    runs = []
+    for _ in range(2):
+        out, cache = net.forward(X)
+        loss, d = net.loss_grad(out, y)
+        runs.append([out, cache[1], cache[2], loss, d] + net.backward(d, cache))
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+    W1, b1, W2, b2, W3, b3 = [p.double() for p in net.params]
+    out, H1, H2, loss, d = [t.double() for t in runs[0][:5]]
+    want = {}
+    want["H1"] = (torch.relu(X.double() @ W1 + b1), H1)
+    want["H2"] = (torch.relu(H1 @ W2 + b2), H2)
+    want["out"] = (H2 @ W3 + b3, out)
+    want["loss"] = (((out - y.double()) ** 2).mean().reshape(1), loss)
+    want["d"] = (2 * (out - y.double()) / rows, d)
+    d2 = (d @ W3.T) * (H2 > 0)
+    d1 = (d2 @ W2.T) * (H1 > 0)
+    refs = [X.double().T @ d1, d1.sum(0), H1.T @ d2, d2.sum(0), H2.T @ d, d.sum(0)]
+    want.update({f"grad{k}": (r, g.double()) for k, (r, g) in enumerate(zip(refs, runs[0][5:]))})
+    for k, (w, got) in want.items():
+        assert w.shape == got.shape, k
+        assert float((got - w).norm()) <= 1e-5 * float(w.norm()), (k, float((got - w).norm()), float(w.norm()))
+
+
 def test_gradients_match_torch_autograd_fp32():
     import torch
     net = _net(11, 128, 3)

@@ -191,9 +191,15 @@ def _lib():
         lib.ttcb_mlp_mse.argtypes = [P, P, I, P, P, P]
         lib.ttcb_mlp_adam.argtypes = [P, P, P, P, I, F, F, F, F, I, P]
         lib.ttcb_mlp_adam_l2.argtypes = [P, P, P, P, I, F, F, F, F, F, I, P]
+        lib.ttcb_mlp_adam_multi.argtypes = [I, P, P, P, P, P, F, F, F, F, F, I, P]
+        lib.ttcb_mlp_forward.argtypes = [I, I, P, P, P, P, P, P]
+        lib.ttcb_mlp_backward.argtypes = [I, I, P, P, P, P, P, P, P, P]
+        lib.ttcb_mlp_backward_workspace.argtypes = [I, I]
         for n in ("ttcb_mlp_gemm", "ttcb_mlp_relu_grad", "ttcb_mlp_colsum", "ttcb_mlp_mse", "ttcb_mlp_adam",
-                  "ttcb_mlp_adam_l2"):
+                  "ttcb_mlp_adam_l2", "ttcb_mlp_adam_multi", "ttcb_mlp_forward", "ttcb_mlp_backward"):
             getattr(lib, n).restype = ctypes.c_int
+        lib.ttcb_mlp_backward_workspace.restype = ctypes.c_size_t
+        lib._mlp_max_in = lib.ttcb_mlp_passes_max_features()
         lib._mlp_bound = True
     return lib
 
@@ -214,6 +220,10 @@ def gemm(A, B, transA=False, transB=False, bias=None, relu=False, out=None):
                                        B.shape[1], C.data_ptr(), N, bias.data_ptr() if bias is not None else None,
                                        int(relu), _s()))
     return C
+
+
+def _ptrs(tensors):
+    return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
 
 
 class MLP:
@@ -240,7 +250,21 @@ class MLP:
         # further ensemble members (same shape and normalisation); predictions average over all
         self.extra = []
 
+    def _one_launch(self, X) -> bool:
+        """Whether the library's whole-network passes take this input (hidden size 128, features that
+        fit); otherwise the passes go layer by layer."""
+        return (self.hidden == 128 and 0 < self.nin <= _lib()._mlp_max_in and X.shape[0] > 0
+                and X.shape[1] == self.nin and X.is_contiguous() and all(p.is_contiguous() for p in self.params))
+
     def forward(self, X):
+        import torch
+        if self._one_launch(X):
+            n = X.shape[0]
+            buf = torch.empty(n * 257, dtype=torch.float32, device=X.device)
+            H1, H2, out = buf[:n * 128].view(n, 128), buf[n * 128:n * 256].view(n, 128), buf[n * 256:].view(n, 1)
+            _native.check(_lib().ttcb_mlp_forward(n, self.nin, X.data_ptr(), _ptrs(self.params), H1.data_ptr(),
+                                                  H2.data_ptr(), out.data_ptr(), _s()))
+            return out, (X, H1, H2)
         W1, b1, W2, b2, W3, b3 = self.params
         H1 = gemm(X, W1, bias=b1, relu=True)
         H2 = gemm(H1, W2, bias=b2, relu=True)
@@ -252,6 +276,14 @@ class MLP:
         X, H1, H2 = cache
         W1, b1, W2, b2, W3, b3 = self.params
         lib, s = _lib(), _s()
+        if self._one_launch(X) and dout.is_contiguous():
+            n, sizes = X.shape[0], [p.numel() for p in self.params]
+            flat = torch.empty(sum(sizes), dtype=torch.float32, device=X.device)
+            work = torch.empty(lib.ttcb_mlp_backward_workspace(n, self.nin) // 4, dtype=torch.float32, device=X.device)
+            _native.check(lib.ttcb_mlp_backward(n, self.nin, X.data_ptr(), _ptrs(self.params), H1.data_ptr(),
+                                                H2.data_ptr(), dout.data_ptr(), flat.data_ptr(), work.data_ptr(), s))
+            g = flat.split(sizes)
+            return [g[0].view(self.nin, 128), g[1], g[2].view(128, 128), g[3], g[4].view(128, 1), g[5]]
         grads = [None] * 6
         grads[4] = gemm(H2, dout, transA=True)
         grads[5] = torch.empty(1, device="cuda")
@@ -273,17 +305,16 @@ class MLP:
     def loss_grad(self, out, y):
         import torch
         d = torch.empty_like(out)
-        loss = torch.zeros(1, device="cuda")
+        loss = torch.empty(1, device="cuda")
         _native.check(_lib().ttcb_mlp_mse(out.data_ptr(), y.data_ptr(), out.numel(), d.data_ptr(), loss.data_ptr(),
                                           _s()))
         return loss, d
 
     def step(self, grads, lr=1e-3, weight_decay=0.0):
         self.t += 1
-        lib, s = _lib(), _s()
-        for p, g, m, v in zip(self.params, grads, self.m, self.v):
-            _native.check(lib.ttcb_mlp_adam_l2(p.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), p.numel(),
-                                               lr, 0.9, 0.999, 1e-8, weight_decay, self.t, s))
+        n = (ctypes.c_int * len(self.params))(*[p.numel() for p in self.params])
+        _native.check(_lib().ttcb_mlp_adam_multi(len(self.params), _ptrs(self.params), _ptrs(grads), _ptrs(self.m),
+                                                 _ptrs(self.v), n, lr, 0.9, 0.999, 1e-8, weight_decay, self.t, _s()))
 
     # -- normalisation and I/O ------------------------------------------------------------------
     def _norm(self, X: np.ndarray):
