@@ -190,7 +190,7 @@ ttcb_status ttcb_batch_create(ttcb_batch** batch, int count, const ttcb_plan* co
 /* Runs every problem of the batch in one persistent kernel launch on stream. */
 ttcb_status ttcb_batch_launch(ttcb_batch* batch, ttcb_stream_t stream);
 
-/* Captures the batch launch (counter reset + kernel) into a CUDA graph once and replays it. */
+/* Captures the batch launch into a CUDA graph once and replays it. */
 ttcb_status ttcb_batch_graph_launch(ttcb_batch* batch, ttcb_stream_t stream);
 
 /* Device status word of the last launch: 0 = ok, otherwise a TTCB_ERR_* code set on the device. */

@@ -104,6 +104,50 @@ def test_batched_ragged_tiles_and_vector_widths(dtype):
         batch.close()
 
 
+@pytest.mark.parametrize("blocks", [1, 3, 0])
+@pytest.mark.parametrize("dtype,beta", [("s", 0.0), ("s", -0.5), ("z", 0.0), ("z", 1.2), ("ds", 0.0)])
+def test_batched_segments(dtype, beta, blocks):
+    """The batch's segments: problems of many tiles (several segments), of one, of ragged tiles moved by
+    vectors, by elements and as edge plans, of rows, and empty ones; tiles from the smallest to 8192
+    elements (rings of one stage up to the deepest), misaligned buffers, few CTAs (segments claimed from
+    the counter) and many; launched three times (the counter is back at zero each time), bit for bit
+    against the oracle."""
+    import torch
+    from ttc_b200 import Plan
+    from ttc_b200.batched import Batch
+    ta, tb = (dtype[0], dtype[1]) if len(dtype) == 2 else (dtype, dtype)
+    shapes = [([1, 0], [64, 640]), ([1, 0], [65, 129]), ([2, 0, 1], [67, 31, 53]), ([0, 2, 1], [300, 5, 7]),
+              ([1, 0, 2], [36, 68, 5]), ([0, 1], [4000, 3]), ([2, 1, 0], [11, 2, 1093]), ([1, 0], [3, 2]),
+              ([1, 0], [0, 5]), ([1, 0], [130, 257])]
+    plans, As, Bs, wants, keep = [], [], [], [], []
+    for k, (perm, size) in enumerate(shapes):
+        for tu in ({}, {"tile_elems": 8192}, {"tile_elems": 256}, {"ragged": 1}):
+            n = int(np.prod(size))
+            a, b = uniform(max(n, 1), ta, 7 * k + 1)[:n], uniform(max(n, 1), tb, 7 * k + 2)[:n]
+            want = b.copy()
+            for _ in range(3):
+                if n:
+                    want = oracle.transpose(a, want, perm, size, 1.5, beta, dtype=dtype)
+            wants.append(want)
+            plans.append(Plan(perm, size, dtype, beta != 0, tuning=tu))
+            off = len(plans) % 3
+            x = torch.from_numpy(np.concatenate([uniform(4, ta, 3)[:off], a])).cuda()
+            y = torch.from_numpy(np.concatenate([uniform(4, tb, 4)[:off], b, uniform(8, tb, 5)])).cuda()
+            keep.append((x, y, off, n))
+            As.append(x[off:])
+            Bs.append(y[off:])
+    batch = Batch(plans, As, Bs, alpha=1.5, beta=beta, blocks=blocks)
+    for _ in range(3):
+        batch.launch(graph=blocks == 0)
+    batch.check_status()
+    torch.cuda.synchronize()
+    for k, ((x, y, off, n), w) in enumerate(zip(keep, wants)):
+        got = y.cpu().numpy()
+        assert_bitexact(got[off:off + n], w, f"problem {k} {plans[k].describe()}")
+        assert_bitexact(got[off + n:], uniform(8, tb, 5), f"past problem {k}")
+    batch.close()
+
+
 def test_batch_rejects_mixed_types():
     from ttc_b200 import Plan, TTCError
     from ttc_b200.batched import Batch

@@ -13,7 +13,7 @@ from .core import Plan, _ptr, _stream_handle, pack_scalar
 class Batch:
     """``Batch(plans, As, Bs, alpha, beta)`` binds device buffers to plans (same dtype pair and beta
     flag for all). ``launch()`` runs every problem in one launch; ``launch(graph=True)`` captures the
-    launch (counter reset + kernel) into a CUDA graph once and replays it."""
+    launch into a CUDA graph once and replays it."""
 
     def __init__(self, plans: Sequence[Plan], As, Bs, alpha=1.0, beta=0.0, blocks: int = 0):
         if not plans:

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <new>
 #include <string>
@@ -46,17 +47,14 @@ struct ttcb_batch {
   unsigned char alpha[16] = {0};
   unsigned char beta[16] = {0};
   int64_t bytes = 0;
-  unsigned long long total = 0;
+  unsigned int nseg = 0;
   int blocks = 0;
-  int smem = 0;         // the stage buffers + the largest problem's tables
-  int slots_bytes = 0;  // one stage buffer (the largest staged tile)
-  int chunk = 1;        // items claimed per atomic
-  void* d_probs = nullptr;
-  int64_t* d_prefix = nullptr;
-  unsigned char* d_desc = nullptr;
-  unsigned long long* d_counter = nullptr;  // [0] next item, [1] status word (as int)
-  cudaGraphExec_t graph_exec = nullptr;
+  int smem = 0;                       // the ring (or a ragged tile's stage and tables)
+  void* d_segs = nullptr;             // ttcb::BatchSeg[nseg]
+  unsigned char* d_desc = nullptr;    // the problems' descriptors
+  unsigned int* d_counter = nullptr;  // segments claimed, CTAs finished, status
   cudaGraph_t graph = nullptr;
+  cudaGraphExec_t graph_exec = nullptr;
   cudaStream_t capture_stream = nullptr;
 };
 
@@ -75,8 +73,7 @@ static void batch_free(ttcb_batch* b) {
   if (b->graph_exec) cudaGraphExecDestroy(b->graph_exec);
   if (b->graph) cudaGraphDestroy(b->graph);
   if (b->capture_stream) cudaStreamDestroy(b->capture_stream);
-  if (b->d_probs) cudaFree(b->d_probs);
-  if (b->d_prefix) cudaFree(b->d_prefix);
+  if (b->d_segs) cudaFree(b->d_segs);
   if (b->d_desc) cudaFree(b->d_desc);
   if (b->d_counter) cudaFree(b->d_counter);
   delete b;
@@ -111,14 +108,12 @@ ttcb_status ttcb_batch_create(ttcb_batch** out, int count, const ttcb_plan* cons
   if (p0->beta_nonzero) std::memcpy(b->beta, beta, EB);
 
   // Problems of the batch: every plan, and for a plan whose ragged tiles its edge plans move, those
-  // edge plans as problems of their own (offset into the plan's A and B) while the plan keeps only
-  // its complete tiles.
+  // edge plans as problems of their own (offset into the plan's A and B).
   struct Entry {
     const ttcb_plan* p;
     const void* A;
     void* B;
-    int full_only;  // the plan's complete tiles only (its edge plans follow it)
-    int user;       // index of the caller's plan
+    int edges;      // its ragged tiles are problems of their own (the edge plans that follow it)
     int own;        // 1: the caller's plan itself (0: one of its edge plans)
   };
   std::vector<Entry> ent;
@@ -141,12 +136,12 @@ ttcb_status ttcb_batch_create(ttcb_batch** out, int count, const ttcb_plan* cons
       batch_free(b);
       return bfail(TTCB_ERR_INVALID_ARG, "A or B of problem " + std::to_string(i) + " is NULL");
     }
-    const bool edges = !p->empty && p->kernel == TTCB_KERNEL_TILE && p->nedge > 0;
-    ent.push_back({p, A[i], B[i], edges ? 1 : 0, i, 1});
+    const bool edges = !p->empty && p->kernel == TTCB_KERNEL_TILE && p->nedge > 0 && !p->rag_inline;
+    ent.push_back({p, A[i], B[i], edges ? 1 : 0, 1});
     for (int k = 0; edges && k < p->nedge; ++k) {
       const ttcb_plan* q = p->edge[k];
       ent.push_back({q, static_cast<const char*>(A[i]) + q->base_offA * EA,
-                     static_cast<char*>(B[i]) + q->base_offB * EB, 0, i, 0});
+                     static_cast<char*>(B[i]) + q->base_offB * EB, 0, 0});
     }
   }
   // The batched kernel stages A in the plain layout (element p at p + (p / sigmaA) * padA); a plan
@@ -206,72 +201,69 @@ ttcb_status ttcb_batch_create(ttcb_batch** out, int count, const ttcb_plan* cons
     }
   }
   std::vector<unsigned char> hdesc(std::max<int64_t>(desc_bytes, 16), 0);
-  std::vector<ttcb::BatchProblem> hp(n);
-  std::vector<int64_t> prefix(n + 1, 0);
-  int max_slots_bytes = 0, max_table_bytes = 0;
+  const bool beta_nz = b->beta_nonzero != 0;
+  // One record per problem, then its segments: runs of at most kSegTiles tiles of about target bytes
+  // (set below, once the grid is known).
+  std::vector<ttcb::BatchSeg> prob(n);
+  int max_stage = 0, max_ragged = 0;
   for (int i = 0; i < n; ++i) {
     const ttcb_plan* p = ent[i].p;
-    ttcb::BatchProblem& q = hp[i];
+    ttcb::BatchSeg& q = prob[i];
     std::memset(&q, 0, sizeof(q));
-    int64_t items = 0;
-    if (!p->empty) {
-      std::memcpy(hdesc.data() + desc_off[i], p->host_desc.data(), p->host_desc.size());
-      q.A = ent[i].A;
-      q.B = ent[i].B;
-      q.kind = p->kernel;
-      q.va = p->vecA;
-      q.vb = p->vecB;
-      q.full_only = ent[i].full_only;
-      while (q.va > 1 && (uintptr_t)q.A % (q.va * EA)) q.va /= 2;
-      while (q.vb > 1 && (uintptr_t)q.B % (q.vb * EB)) q.vb /= 2;
-      if (p->kernel == TTCB_KERNEL_ROW) {
-        q.va = q.vb = std::min(q.va, q.vb);
-        const RowDesc* rd = reinterpret_cast<const RowDesc*>(p->host_desc.data());
-        items = (rd->nunits + 7) / 8;
-      } else {
-        const TileDesc* td = reinterpret_cast<const TileDesc*>(p->host_desc.data());
-        items = ent[i].full_only ? td->nfull : td->ntiles;
-        // one stage buffer: the staged layout (or, for a ragged tile, the slots), 16-byte aligned
-        max_slots_bytes = std::max<int>(
-            max_slots_bytes, (int)ttcb::al16((size_t)std::max(td->stage_elems, td->phys_size) * EA));
-        max_table_bytes = std::max<int>(max_table_bytes, 8 * (td->nsegA + td->nsegB) + 4 * ((td->P + 1) / 2));
-      }
-      if (ent[i].own) b->bytes += ttcb_plan_bytes(p);  // an edge plan's bytes are its parent's
+    if (p->empty) continue;
+    std::memcpy(hdesc.data() + desc_off[i], p->host_desc.data(), p->host_desc.size());
+    q.A = ent[i].A;
+    q.B = ent[i].B;
+    q.desc = reinterpret_cast<const unsigned char*>((uintptr_t)desc_off[i]);  // its offset, until the upload
+    q.va = p->vecA;
+    q.vb = p->vecB;
+    while (q.va > 1 && (uintptr_t)q.A % (q.va * EA)) q.va /= 2;
+    while (q.vb > 1 && (uintptr_t)q.B % (q.vb * EB)) q.vb /= 2;
+    if (ent[i].own) b->bytes += ttcb_plan_bytes(p);  // an edge plan's bytes are its parent's
+    if (p->kernel == TTCB_KERNEL_ROW) {
+      q.kind = ttcb::kSegRows;
+      q.va = q.vb = std::min(q.va, q.vb);
+      continue;
     }
-    prefix[i + 1] = prefix[i] + items;
+    const TileDesc* td = reinterpret_cast<const TileDesc*>(p->host_desc.data());
+    q.kind = ttcb::kSegFull;
+    q.rag_vec = p->rag_inline == ttcb::kRagVec;
+    q.P = td->P;
+    q.LA = td->LA;
+    q.LB = td->LB;
+    q.padA = td->padA;
+    q.a_bytes = (int)ttcb::al16((size_t)td->stage_elems * EA);
+    q.stage_bytes = (int)ttcb::async_stage_bytes(td->stage_elems, td->P, EA, EB, beta_nz);
+    q.off_segA = td->off_segA;
+    q.off_segB = td->off_segB;
+    q.off_gtab = td->off_gtab;
+    // (the access widths actually used: half or scalar widths where the kernel has no third)
+    const int wa = q.va * EA == 16 ? q.va : q.va * EA == 8 && EA < 8 ? q.va : 1;
+    const int wb = q.vb * EB == 16 ? q.vb : q.vb * EB == 8 && EB < 8 ? q.vb : 1;
+    q.reg = td->reg_ok && td->P / wa <= 4 * ttcb::kThreads && td->P / wb <= 4 * ttcb::kThreads;
+    q.ng = td->ngrid;
+    q.divLA = td->divLA;
+    q.divLB = td->divLB;
+    q.divSigma = td->divSigmaA;
+    for (int g = 0; g < td->ngrid; ++g) {
+      q.g[g].div = td->g[g].divf;
+      q.g[g].sA = td->g[g].strideA;
+      q.g[g].sB = td->g[g].strideB;
+    }
+    max_stage = std::max(max_stage, q.stage_bytes);
+    if (!ent[i].edges && td->nrag0 + td->nrag1 > 0)
+      max_ragged = std::max(max_ragged, q.stage_bytes + 8 * (td->nsegA + td->nsegB) + 4 * ((td->P + 1) / 2));
   }
-  b->total = (unsigned long long)prefix[n];
-  b->slots_bytes = (int)((max_slots_bytes + 15) & ~15);
-  b->smem = ttcb::kBatchStages * b->slots_bytes + max_table_bytes;  // stage buffers, then the tables
-
-  // device copies
-  if ((e = cudaMalloc(&b->d_desc, hdesc.size())) != cudaSuccess ||
-      (e = cudaMalloc(&b->d_probs, sizeof(ttcb::BatchProblem) * n)) != cudaSuccess ||
-      (e = cudaMalloc(&b->d_prefix, sizeof(int64_t) * (n + 1))) != cudaSuccess ||
-      (e = cudaMalloc(&b->d_counter, 2 * sizeof(unsigned long long))) != cudaSuccess) {
-    cudaGetLastError();
-    batch_free(b);
-    return bfail(TTCB_ERR_ALLOC, std::string("cudaMalloc for the batch failed: ") + cudaGetErrorString(e));
-  }
-  for (int i = 0; i < n; ++i)
-    if (desc_off[i] >= 0) hp[i].desc = b->d_desc + desc_off[i];
-  if ((e = cudaMemcpy(b->d_desc, hdesc.data(), hdesc.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(b->d_probs, hp.data(), sizeof(ttcb::BatchProblem) * n, cudaMemcpyHostToDevice)) !=
-          cudaSuccess ||
-      (e = cudaMemcpy(b->d_prefix, prefix.data(), sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice)) !=
-          cudaSuccess ||
-      (e = cudaMemset(b->d_counter, 0, 2 * sizeof(unsigned long long))) != cudaSuccess) {
-    batch_free(b);
-    return bcuda(e, "batch descriptor upload");
-  }
-
+  // The ring: what lets batch_min_blocks CTAs share an SM (227 KB less 1 KB and about 2.6 KB of static shared
+  // memory per CTA), more where a tile needs it. At 1024 fp32 problems it holds three stages or more of
+  // nine tiles in ten.
+  b->smem = std::max({beta_nz ? 72 * 1024 : 52 * 1024, (max_stage + 15) & ~15, (max_ragged + 15) & ~15});
   ttcb::BatchKernelRef k = ttcb::pick_batch_kernel(b->ta, b->tb, batch_variant(b));
   if (!k.func) {
     batch_free(b);
     return bfail(TTCB_ERR_DTYPE, "no batched kernel for this type pair");
   }
-  if (b->smem + (int)sizeof(TileDesc) + 64 > 48 * 1024)  // + its static header copy, item and problem index
-    ttcb::allow_large_smem(k.func);
+  ttcb::allow_large_smem(k.func);
   int sms = 0, per_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.func, ttcb::kThreads, b->smem);
@@ -279,25 +271,84 @@ ttcb_status ttcb_batch_create(ttcb_batch** out, int count, const ttcb_plan* cons
     batch_free(b);
     return e != cudaSuccess ? bcuda(e, "occupancy query") : bfail(TTCB_ERR_UNSUPPORTED, "batch tile too large");
   }
-  int64_t resident = (int64_t)per_sm * sms;
-  int64_t nb = blocks > 0 ? blocks : resident;
-  nb = std::min<int64_t>(nb, std::max<unsigned long long>(b->total, 1ull));
-  b->blocks = (int)std::max<int64_t>(nb, 1);
-  // about sixteen claims per CTA keep the tail balanced while amortising the claim and its search
-  b->chunk = (int)std::max<unsigned long long>(1ull, std::min<unsigned long long>(
-                                                         32ull, b->total / (16ull * (unsigned long long)b->blocks)));
+  const int64_t most = blocks > 0 ? blocks : (int64_t)per_sm * sms;
+  // About twelve segments per CTA, at most 128 KB: fewer and longer ones leave the CTAs on more problems at
+  // once, far apart in memory, and a longer tail (1024 problems of 105 Ki elements: 284 us with twelve,
+  // 296 with eight, 334 with four; 303 with 24)
+  const int64_t target = std::min<int64_t>(std::max<int64_t>(b->bytes / (12 * most), 16 * 1024), 128 * 1024);
+  std::vector<ttcb::BatchSeg> segs;
+  std::vector<std::pair<int64_t, uint32_t>> order;  // (key, segment): largest first
+  const int64_t elem = EA + EB * (beta_nz ? 2 : 1);
+  auto cut = [&](const ttcb::BatchSeg& q, int kind, int64_t items, int64_t item_bytes, int limit) {
+    const int64_t per = std::min<int64_t>(std::max<int64_t>(target / std::max<int64_t>(item_bytes, 1), 1), limit);
+    const int64_t pieces = (items + per - 1) / per;
+    for (int64_t j = 0, t = 0; j < pieces; ++j) {
+      const int64_t m = (items - t + (pieces - j) - 1) / (pieces - j);
+      ttcb::BatchSeg s = q;
+      s.kind = kind;
+      s.t0 = (uint32_t)t;
+      s.nt = (int32_t)m;
+      const int64_t weight = m * item_bytes + 8192;  // (a segment's start costs about as much as 8 KB)
+      const int64_t bucket = (int64_t)(2.0 * std::log2((double)weight));
+      order.push_back({-(bucket * 1024 + kind * 256 + q.va * 16 + q.vb), (uint32_t)segs.size()});
+      segs.push_back(s);
+      t += m;
+    }
+  };
+  for (int i = 0; i < n; ++i) {
+    const ttcb_plan* p = ent[i].p;
+    if (p->empty) continue;
+    ttcb::BatchSeg& q = prob[i];
+    if (q.kind == ttcb::kSegRows) {
+      const RowDesc* rd = reinterpret_cast<const RowDesc*>(p->host_desc.data());
+      cut(q, ttcb::kSegRows, (rd->nunits + 7) / 8, 8 * (int64_t)rd->chunk * elem, 1 << 20);
+      continue;
+    }
+    const TileDesc* td = reinterpret_cast<const TileDesc*>(p->host_desc.data());
+    q.stages = std::min(b->smem / q.stage_bytes, ttcb::kMaxStages);
+    cut(q, ttcb::kSegFull, td->nfull, td->P * elem, ttcb::kSegTiles);
+    if (!ent[i].edges) cut(q, ttcb::kSegRagged, (int64_t)td->nrag0 + td->nrag1, 4 * td->P * elem, 1 << 20);
+  }
+  if (segs.size() >= (size_t)1 << 30) {
+    batch_free(b);
+    return bfail(TTCB_ERR_UNSUPPORTED, "batch too large");
+  }
+  // The largest segments first, so that the last ones claimed are small; among segments of a size those
+  // of one access width together (CTAs of an SM then share their instructions).
+  std::stable_sort(order.begin(), order.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
+  {
+    std::vector<ttcb::BatchSeg> sorted;
+    sorted.reserve(segs.size());
+    for (const auto& o : order) sorted.push_back(segs[o.second]);
+    segs.swap(sorted);
+  }
+  b->nseg = (unsigned int)segs.size();
+  b->blocks = (int)std::max<int64_t>(std::min<int64_t>(most, b->nseg), 1);
+
+  // device copies
+  if ((e = cudaMalloc(&b->d_desc, hdesc.size())) != cudaSuccess ||
+      (e = cudaMalloc(&b->d_segs, sizeof(ttcb::BatchSeg) * std::max<size_t>(segs.size(), 1))) != cudaSuccess ||
+      (e = cudaMalloc(&b->d_counter, 4 * sizeof(unsigned int))) != cudaSuccess) {
+    cudaGetLastError();
+    batch_free(b);
+    return bfail(TTCB_ERR_ALLOC, std::string("cudaMalloc for the batch failed: ") + cudaGetErrorString(e));
+  }
+  for (ttcb::BatchSeg& s : segs) s.desc = b->d_desc + reinterpret_cast<uintptr_t>(s.desc);
+  if ((e = cudaMemcpy(b->d_desc, hdesc.data(), hdesc.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
+      (!segs.empty() && (e = cudaMemcpy(b->d_segs, segs.data(), sizeof(ttcb::BatchSeg) * segs.size(),
+                                        cudaMemcpyHostToDevice)) != cudaSuccess) ||
+      (e = cudaMemset(b->d_counter, 0, 4 * sizeof(unsigned int))) != cudaSuccess) {
+    batch_free(b);
+    return bcuda(e, "batch descriptor upload");
+  }
   *out = b;
   return TTCB_OK;
 }
 
 static ttcb_status batch_enqueue(ttcb_batch* b, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned long long), s);
-  if (e != cudaSuccess) return bcuda(e, "counter reset");
-  if (b->total == 0) return TTCB_OK;
+  if (b->nseg == 0) return TTCB_OK;
   ttcb::BatchKernelRef k = ttcb::pick_batch_kernel(b->ta, b->tb, batch_variant(b));
-  e = k.fn(b->d_probs, b->d_prefix, b->count, b->total, b->d_counter,
-           reinterpret_cast<int*>(b->d_counter + 1), b->alpha, b->beta, b->blocks, b->smem, b->slots_bytes,
-           b->chunk, s);
+  cudaError_t e = k.fn(b->d_segs, b->nseg, b->d_counter, b->alpha, b->beta, b->blocks, b->smem, s);
   if (e != cudaSuccess) return bcuda(e, "batched kernel launch");
   return TTCB_OK;
 }
@@ -309,6 +360,7 @@ ttcb_status ttcb_batch_launch(ttcb_batch* b, ttcb_stream_t stream) {
 
 ttcb_status ttcb_batch_graph_launch(ttcb_batch* b, ttcb_stream_t stream) {
   if (!b) return bfail(TTCB_ERR_INVALID_ARG, "batch is NULL");
+  if (b->nseg == 0) return TTCB_OK;
   cudaError_t e;
   if (!b->graph_exec) {
     // capture once on a private stream (the legacy default stream cannot be captured)
@@ -338,7 +390,7 @@ ttcb_status ttcb_batch_graph_launch(ttcb_batch* b, ttcb_stream_t stream) {
 ttcb_status ttcb_batch_status(ttcb_batch* b, ttcb_stream_t stream) {
   if (!b) return bfail(TTCB_ERR_INVALID_ARG, "batch is NULL");
   int st = 0;
-  cudaError_t e = cudaMemcpyAsync(&st, b->d_counter + 1, sizeof(int), cudaMemcpyDeviceToHost,
+  cudaError_t e = cudaMemcpyAsync(&st, b->d_counter + 2, sizeof(int), cudaMemcpyDeviceToHost,
                                   reinterpret_cast<cudaStream_t>(stream));
   if (e == cudaSuccess) e = cudaStreamSynchronize(reinterpret_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return bcuda(e, "batch status read");

@@ -610,25 +610,23 @@ __device__ __forceinline__ bool ragged_in(const TileDesc& d, uint32_t p, int lim
   return ok;
 }
 
-// The CTA's ragged tiles (see kRagVec), V = VA (VB) elements at a time, in two of the S stages at `smem`
-// (sbytes each; the B tile a_bytes in). The tables go to shared memory (run tables behind the stages,
-// the gather table in the third stage) and the first tile is decoded before the previous launch is
-// waited for: a small call's time is the latency of its one ragged tile, and with the tables read from
-// global memory after the wait 46 tiles of fp64 took 6.2 us. Two entries of info are used. Ends
+// Ragged tiles r, r + step, .. below R of a tile problem (see kRagVec), V = VA (VB) elements at a time, in
+// nbuf (1 or 2) stages at `smem` (sbytes each; the B tile a_bytes in). The tables go to shared memory (run
+// tables at segA, the gather table at gtab) and the first tile is decoded before the previous launch
+// is waited for: a small call's time is the latency of its one ragged tile, and with the tables read from
+// global memory after the wait 46 tiles of fp64 took 6.2 us (so 5.5). nbuf entries of info are used. Ends
 // with every thread done with the stages.
 template <typename TA, typename TB, int VA, int VB, bool BETA, bool STREAM>
 __device__ __noinline__ void ragged_pass(const TileDesc& d, const unsigned char* desc, const TA* __restrict__ A,
                                          TB* __restrict__ B, TA alpha, TB beta, unsigned char* smem, uint32_t a_bytes,
-                                         uint32_t sbytes, TileInfo* info, int a0) {
+                                         uint32_t sbytes, int64_t* segA, uint16_t* gtab, TileInfo* info, int a0,
+                                         int nbuf, uint32_t r, uint32_t R, uint32_t step) {
   constexpr int VM = 16 / (int)sizeof(TA);
   const int P = d.P, LA = d.LA, LB = d.LB, nsegA = d.nsegA, nsegB = d.nsegB;
-  const uint32_t R = (uint32_t)(d.nrag0 + d.nrag1), G = gridDim.x;
-  int64_t* segA = reinterpret_cast<int64_t*>(smem + d.nstages * sbytes);
   int64_t* segB = segA + nsegA;
-  uint16_t* gtab = reinterpret_cast<uint16_t*>(smem + 2 * sbytes);
-  auto decode = [&](uint32_t r, TileInfo& ti) {
+  auto decode = [&](uint32_t t, TileInfo& ti) {
     int lim[2];
-    decode_tile(d, ragged_tile_index(d, r), ti.bA, ti.bB, lim);
+    decode_tile(d, ragged_tile_index(d, t), ti.bA, ti.bB, lim);
     ti.lim0 = lim[0];
     ti.lim1 = lim[1];
   };
@@ -663,15 +661,14 @@ __device__ __noinline__ void ragged_pass(const TileDesc& d, const unsigned char*
     for (int i = threadIdx.x; i < nsegB; i += kThreads) segB[i] = gB[i];
     for (int i = threadIdx.x; i < (P + 1) / 2; i += kThreads) reinterpret_cast<uint32_t*>(gtab)[i] = gG[i];
   }
-  uint32_t r = blockIdx.x;
   if (threadIdx.x == 0) decode(r, info[0]);
   __syncthreads();
   pdl_wait_previous();
   issue(info[0], 0);
-  for (uint32_t cur = 0;; cur ^= 1) {
-    const uint32_t rn = r + G;
+  for (uint32_t cur = 0;; cur = nbuf == 2 ? cur ^ 1 : 0) {
+    const uint32_t rn = r + step;
     const bool more = rn < R;
-    if (more) {
+    if (more && nbuf == 2) {
       if (threadIdx.x == 0) decode(rn, info[cur ^ 1]);
       __syncthreads();  // also: every thread is done with the other stage
       issue(info[cur ^ 1], cur ^ 1);
@@ -702,6 +699,11 @@ __device__ __noinline__ void ragged_pass(const TileDesc& d, const unsigned char*
     if (!more) break;
     r = rn;
     __syncthreads();
+    if (nbuf != 2) {
+      if (threadIdx.x == 0) decode(r, info[0]);
+      __syncthreads();
+      issue(info[0], 0);
+    }
   }
   // a bulk copy may follow these generic-proxy writes into a stage
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -757,10 +759,14 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
   const uint16_t* ggtab = reinterpret_cast<const uint16_t*>(base + d.off_gtab);
   const uint32_t nrag = rag ? (uint32_t)(d.nrag0 + d.nrag1) : 0u;
   if (blockIdx.x < nrag) {
+    int64_t* tabs = reinterpret_cast<int64_t*>(smem_raw + S * sbytes);
+    uint16_t* gt = reinterpret_cast<uint16_t*>(smem_raw + 2 * sbytes);  // the third stage
     if (rag == kRagVec)
-      ragged_pass<TA, TB, VA, VB, BETA, STREAM>(d, base, A, B, alpha, beta, smem_raw, a_bytes, sbytes, info, a0);
+      ragged_pass<TA, TB, VA, VB, BETA, STREAM>(d, base, A, B, alpha, beta, smem_raw, a_bytes, sbytes, tabs, gt, info,
+                                                a0, 2, blockIdx.x, nrag, gridDim.x);
     else
-      ragged_pass<TA, TB, 1, 1, BETA, STREAM>(d, base, A, B, alpha, beta, smem_raw, a_bytes, sbytes, info, a0);
+      ragged_pass<TA, TB, 1, 1, BETA, STREAM>(d, base, A, B, alpha, beta, smem_raw, a_bytes, sbytes, tabs, gt, info, a0,
+                                              2, blockIdx.x, nrag, gridDim.x);
   }
   {
     const int64_t* gA = reinterpret_cast<const int64_t*>(base + d.off_segA);

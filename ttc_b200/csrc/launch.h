@@ -34,9 +34,8 @@ bool needs_large_smem(int dynamic_smem);
 // never lowers it. Every entry point that launches a kernel goes through this (defined in abi.cu).
 void allow_large_smem(const void* func);
 
-using BatchLaunchFn = cudaError_t (*)(const void* probs, const int64_t* prefix, int count, unsigned long long total,
-                                      unsigned long long* counter, int* status, const void* alpha, const void* beta,
-                                      int blocks, int smem, int slots_bytes, int chunk, cudaStream_t stream);
+using BatchLaunchFn = cudaError_t (*)(const void* segs, unsigned int nseg, unsigned int* counter, const void* alpha,
+                                      const void* beta, int blocks, int smem, cudaStream_t stream);
 struct BatchKernelRef {
   BatchLaunchFn fn = nullptr;
   const void* func = nullptr;
