@@ -6,6 +6,7 @@ only. All arithmetic happens in the sm_100a kernels of ``libttcb200.so``.
 from __future__ import annotations
 
 import ctypes
+import functools
 import json
 from typing import Optional, Sequence
 
@@ -25,12 +26,17 @@ def split_dtype(dtype: str):
     return (dtype[0], dtype[1]) if len(dtype) == 2 else (dtype, dtype)
 
 
+_LETTER_OF_TORCH: dict = {}
+
+
 def torch_letter(t) -> str:
-    import torch
-    m = {torch.float32: "s", torch.float64: "d", torch.complex64: "c", torch.complex128: "z"}
-    if t.dtype not in m:
+    if not _LETTER_OF_TORCH:
+        import torch
+        _LETTER_OF_TORCH.update({torch.float32: "s", torch.float64: "d", torch.complex64: "c", torch.complex128: "z"})
+    letter = _LETTER_OF_TORCH.get(t.dtype)
+    if letter is None:
         raise TTCError(5, f"unsupported tensor dtype {t.dtype}")
-    return m[t.dtype]
+    return letter
 
 
 def pack_scalar(letter: str, value) -> ctypes.Array:
@@ -49,6 +55,19 @@ def pack_scalar(letter: str, value) -> ctypes.Array:
     return (ctypes.c_double * 2)(v.real, v.imag)
 
 
+@functools.lru_cache(maxsize=256)
+def _packed_real(letter: str, value: float) -> ctypes.Array:
+    return pack_scalar(letter, value)
+
+
+def packed(letter: str, value) -> ctypes.Array:
+    """pack_scalar's array (not to be written to); those of nonzero Python floats and ints are shared.
+    (Zeros and complex values are not: equal ones may differ in a zero's sign.)"""
+    if value and (type(value) is float or type(value) is int):
+        return _packed_real(letter, float(value))
+    return pack_scalar(letter, value)
+
+
 def _ptr(x) -> int:
     if isinstance(x, int):
         return x
@@ -59,10 +78,24 @@ def _ptr(x) -> int:
     raise TTCError(1, f"cannot take a device pointer of {type(x)}")
 
 
+_raw_stream = None
+
+
+def current_stream_handle() -> int:
+    """The handle of torch's current stream on the current device (0.3 us; building torch's stream object
+    takes 2.7)."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        torch.cuda.current_stream()  # initialises CUDA
+        get, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), torch.cuda.current_device
+        _raw_stream = (lambda: get(dev())) if get else (lambda: torch.cuda.current_stream().cuda_stream)
+    return _raw_stream()
+
+
 def _stream_handle(stream) -> Optional[int]:
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        return current_stream_handle()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
@@ -103,13 +136,15 @@ class Plan:
         """Launches the transposition on ``stream`` (default: torch's current stream). Asynchronous."""
         if self._h.value is None:
             raise TTCError(1, "plan was destroyed")
-        if complex(beta) != 0 and not self.beta_nonzero:
-            raise TTCError(11, "plan was created for beta == 0")
-        al = pack_scalar(self.ta, alpha)
-        be = pack_scalar(self.tb, beta) if self.beta_nonzero else None
-        check(lib().ttcb_transpose(self._h, _ptr(A), _ptr(B), ctypes.cast(al, ctypes.c_void_p),
-                                   ctypes.cast(be, ctypes.c_void_p) if be is not None else None,
-                                   _stream_handle(stream)))
+        if not self.beta_nonzero:
+            if complex(beta) != 0:
+                raise TTCError(11, "plan was created for beta == 0")
+            be = None
+        else:
+            be = packed(self.tb, beta)
+        status = lib().ttcb_transpose(self._h, _ptr(A), _ptr(B), packed(self.ta, alpha), be, _stream_handle(stream))
+        if status:
+            check(status)
 
     def describe(self) -> dict:
         n = lib().ttcb_plan_describe(self._h, None, 0)
@@ -160,7 +195,7 @@ def transpose(A, B, perm: Sequence[int], size: Optional[Sequence[int]] = None, a
     if tb != dtype:
         dtype = dtype + tb
     key = (tuple(perm), tuple(size), dtype, complex(beta) != 0, tuple(lda or ()), tuple(ldb or ()),
-           tuple(sorted((k, tuple(v) if isinstance(v, list) else v) for k, v in (tuning or {}).items())),
+           tuple(sorted((k, tuple(v) if isinstance(v, list) else v) for k, v in tuning.items())) if tuning else (),
            A.device.index)
     plan = _plan_cache.get(key)
     if plan is None:

@@ -30,7 +30,7 @@ import numpy as np
 
 from . import _native
 from .autotune import Problem, candidate_tunings, measure, Bench, staged_claims
-from .core import ELEM_BYTES, plan_shapes, split_dtype
+from .core import ELEM_BYTES, current_stream_handle, plan_shapes, split_dtype
 
 MAXD = 6
 DEFAULT_MODEL = Path(__file__).resolve().parent / "data" / "cost_model.npz"
@@ -205,8 +205,7 @@ def _lib():
 
 
 def _s():
-    import torch
-    return torch.cuda.current_stream().cuda_stream
+    return current_stream_handle()
 
 
 def gemm(A, B, transA=False, transB=False, bias=None, relu=False, out=None):

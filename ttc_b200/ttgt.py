@@ -22,6 +22,8 @@ not a path that avoids allocation).
 """
 from __future__ import annotations
 
+import contextlib
+import functools
 import math
 from typing import Optional
 
@@ -56,6 +58,13 @@ def plan_contraction(a: str, b: str, c: str) -> dict:
             "perm_c": [c_mat.index(m) for m in c]}
 
 
+@functools.lru_cache(maxsize=256)
+def _contraction(a: str, b: str, c: str) -> dict:
+    """plan_contraction's result, shared (not to be written to), with whether A and B need no transposition."""
+    p = plan_contraction(a, b, c)
+    return dict(p, a_as_is=p["perm_a"] == list(range(len(a))), b_as_is=p["perm_b"] == list(range(len(b))))
+
+
 def _transpose(src, dst, perm, size, alpha, beta, stream):
     dtype = torch_letter(src)
     key = (tuple(perm), tuple(size), dtype, complex(beta) != 0, src.device.index)
@@ -70,7 +79,7 @@ def contract(A, a: str, B, b: str, C, c: str, extents: dict, alpha=1.0, beta=0.0
     tensors of one dtype (float32, float64, complex64 or complex128), in TTC's column-major layout
     with the extents given per mode. Asynchronous on ``stream`` (default: torch's current stream)."""
     import torch
-    p = plan_contraction(a, b, c)
+    p = _contraction(a, b, c)
     for name, t, s in (("A", A, a), ("B", B, b), ("C", C, c)):
         missing = [m for m in s if m not in extents]
         if missing:
@@ -82,14 +91,14 @@ def contract(A, a: str, B, b: str, C, c: str, extents: dict, alpha=1.0, beta=0.0
         raise TTCError(5, "A, B and C must have one dtype")
     ext = lambda s: [extents[m] for m in s]
     n = lambda s: math.prod(ext(s))
-    st = stream if stream is not None else torch.cuda.current_stream()
-    with torch.cuda.stream(st):
-        if p["perm_a"] == list(range(len(a))):
+    st = stream
+    with torch.cuda.stream(st) if st is not None else contextlib.nullcontext():
+        if p["a_as_is"]:
             Am = A
         else:
             Am = torch.empty_like(A)
             _transpose(A, Am, p["perm_a"], ext(a), 1.0, 0.0, st)
-        if p["perm_b"] == list(range(len(b))):
+        if p["b_as_is"]:
             Bm = B
         else:
             Bm = torch.empty_like(B)
