@@ -357,6 +357,25 @@ def test_ragged_tiles_in_the_staged_launch(dtype, beta):
     assert {k[0] for k in seen} >= {1, 2}, seen
 
 
+@pytest.mark.parametrize("dtype", ["s", "sd", "ds"])
+def test_tiles_of_eight_narrow_accesses_per_thread(dtype):
+    """Problems large enough (64 MB moved) for tiles of up to eight 4-byte accesses per thread on a side,
+    with odd extents that leave such accesses on A, on B or on both, ragged tiles, misaligned pointers,
+    round-robin and claimed tiles, bit for bit against the oracle (beta = 0; with beta the same shapes keep
+    four)."""
+    wide = 0
+    for perm, size in [([1, 0], [27, 300007]), ([1, 0], [300011, 27]), ([1, 0, 2], [99, 17, 4813]),
+                       ([2, 1, 0], [10, 25, 32771])]:
+        for offset, beta, tuning in ((0, 0.0, None), (1, 0.0, None), (0, 0.0, {"round_robin": -1}), (0, -0.5, None)):
+            desc = check_case(perm, size, dtype, 1.5, beta, tuning=tuning, offset=offset)
+            t = desc["tile"]
+            narrow = max(t["P"] // desc["vecA"], t["P"] // desc["vecB"])
+            if t["reg"] == 1:  # (tiles off the register path may be larger)
+                assert narrow <= (2048 if beta == 0 else 1024), desc
+                wide += narrow > 1024
+    assert wide >= 3, wide
+
+
 def test_claimed_tiles_with_concurrent_launches_and_slot_reuse():
     """The staged kernel's tiles claimed from the plan's counters: one plan launched on four streams
     at once (different counter slots), then 150 launches in a row on one stream (every slot used and

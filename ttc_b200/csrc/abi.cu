@@ -265,7 +265,7 @@ static ttcb_status launch_plan(const ttcb_plan* p, const void* A, void* B, const
     if (shifted && !((want == 0 || want == 3) && td->async_ok))
       return fail(TTCB_ERR_UNSUPPORTED, "a plan with shifted A runs runs only on the staged tile kernel");
     if ((want == 0 || want == 3) && td->async_ok) {
-      kernel = staged_kernel_id(p, td, fast_ok && td->reg_ok, uses_bulk(p, td, va, EA));
+      kernel = staged_kernel_id(p, td, td->reg_ok && ttcb::reg_path_fits(td->P, va, EA, vb, EB, p->beta_nonzero != 0), uses_bulk(p, td, va, EA));
       blocks = p->blocks_async;
       smem = p->smem_async;
     } else if ((want == 0 || want == 2) && fast_ok) {

@@ -254,7 +254,7 @@ ttcb_status ttcb_batch_create(ttcb_batch** out, int count, const ttcb_plan* cons
     if (!ent[i].edges && td->nrag0 + td->nrag1 > 0)
       max_ragged = std::max(max_ragged, q.stage_bytes + 8 * (td->nsegA + td->nsegB) + 4 * ((td->P + 1) / 2));
   }
-  // The ring: what lets batch_min_blocks CTAs share an SM (227 KB less 1 KB and about 2.6 KB of static shared
+  // The ring: what lets batch_min_blocks CTAs share an SM (228 KB less 1 KB and about 4 KB of static shared
   // memory per CTA), more where a tile needs it. At 1024 fp32 problems it holds three stages or more of
   // nine tiles in ten.
   b->smem = std::max({beta_nz ? 72 * 1024 : 52 * 1024, (max_stage + 15) & ~15, (max_ragged + 15) & ~15});

@@ -61,7 +61,7 @@ struct TileDesc {
   int32_t sigmaA;     // staged layout: element p at p + (p / sigmaA) * padA
   int32_t reg_ok;     // 1: fast, and the staged tile's byte offsets fit 16 bits (register path)
   // ragged tiles (last block of a blocked dimension that does not divide its extent), which the
-  // staged kernel leaves to the ragged-tile kernel: grid dimensions rag_a, rag_b (-1: none);
+  // staged kernel moves in a pass of its own or leaves to other launches: grid dimensions rag_a, rag_b (-1: none);
   // tiles with rag_a at its last block come first (nrag0), then those with rag_b at its last block
   // and rag_a not (nrag1)
   int32_t rag_a, rag_b, nrag0, nrag1;

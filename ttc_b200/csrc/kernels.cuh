@@ -512,6 +512,15 @@ constexpr int async_min_blocks(int bytes_a, int bytes_b, bool beta) {
   return (beta && bytes_a + bytes_b >= 24) ? 3 : 4;
 }
 constexpr int kRegVec = 4;   // vectors per thread and side whose offsets the register path keeps
+// Of 4-byte accesses the staged kernel keeps eight with beta = 0: with four, a tile of them holds 1024
+// elements, and its barrier and decode cost as much as its elements (200 MiB fp32, 27 x 1941807: 102 us with
+// four, 82 with eight; 23 x 2279513: 114 and 83). With beta != 0 the B stream's registers leave no room for them
+// at four CTAs per SM, and at three they were slower as often as faster (0.86-1.15).
+constexpr int reg_vecs(int access_bytes, bool beta) { return access_bytes == 4 && !beta ? 2 * kRegVec : kRegVec; }
+// Whether P elements, accessed va (vb) at a time, fit the staged kernel's register path.
+constexpr bool reg_path_fits(int64_t P, int va, int ea, int vb, int eb, bool beta) {
+  return P <= (int64_t)va * kThreads * reg_vecs(va * ea, beta) && P <= (int64_t)vb * kThreads * reg_vecs(vb * eb, beta);
+}
 
 // V consecutive 16-bit table entries (V-aligned) in one shared-memory access.
 template <typename T, int V> __device__ __forceinline__ void ld_u16s(const uint16_t* p, uint16_t* out) {
@@ -710,7 +719,7 @@ __device__ __noinline__ void ragged_pass(const TileDesc& d, const unsigned char*
   __syncthreads();
 }
 
-// REG: every tile-relative offset of this thread lives in registers (tiles of at most kRegVec
+// REG: every tile-relative offset of this thread lives in registers (tiles of at most reg_vecs
 // vectors per thread and side whose offsets fit 32 bits and whose staged bytes fit 16 bits): A
 // source offsets rA, staged byte offsets dA (two per register), B offsets rB, gather byte offsets
 // gp (two per register; B vector u = tid + u * kThreads, element j). Otherwise offsets are computed
@@ -785,14 +794,16 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
   const bool shift = VA * sizeof(TA) == 16 && d.shiftA;
   // A copies per tile: VA-element vectors, or with shifted runs the chunk slots of every run
   const int nvA = shift ? d.nsegA * d.shiftCM : P / VA, nvB = P / VB;
-  constexpr int kVecB = REG ? kRegVec : kRegPos / VB;  // B vectors per thread with positions in gp
+  constexpr int NA = reg_vecs(VA * sizeof(TA), BETA), NB = reg_vecs(VB * sizeof(TB), BETA);  // register path's vectors
+  constexpr bool kShift = VA * sizeof(TA) == 16;       // shifted runs are possible
+  constexpr int kVecB = REG ? NB : kRegPos / VB;  // B vectors per thread with positions in gp
   constexpr int kGp = (kVecB * VB + 1) / 2;
   // gather positions: byte offsets in the register path, element positions otherwise
   uint32_t gp[kGp];
-  int32_t rA[REG ? kRegVec : 1], rB[REG ? kRegVec : 1];
-  uint32_t dA[REG ? kRegVec / 2 : 1];
-  // the tile shifts x for which each of the thread's A copies is made: x in [lo, hi), 4-bit fields
-  // (lo + 1, hi) per copy; without shifted runs a copy is made at x = 0 when it exists
+  int32_t rA[REG ? NA : 1], rB[REG ? NB : 1];
+  uint32_t dA[REG ? NA / 2 : 1];
+  // which of the thread's A copies are made: the tile shifts x of each, x in [lo, hi), 4-bit fields
+  // (lo + 1, hi) per copy (without shifted runs x = 0 alone); a bit per copy where there are eight
   uint32_t lohi = 0;
   // the register path's lane map (TileDesc::map_log2s): the B vector of thread slot i
   const bool lane_map = REG && d.map_log2s >= 0 && d.map_vb == VB;
@@ -808,7 +819,7 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
   };
   uint32_t vmask = 0;  // register path: bit u set when the thread's slot u takes a B vector
   // BETA, register path: the B stage byte offset of each of the thread's B vectors (two per register)
-  uint32_t qb[REG && BETA ? (kRegVec + 1) / 2 : 1];
+  uint32_t qb[REG && BETA ? (NB + 1) / 2 : 1];
 #pragma unroll
   for (int e = 0; e < (int)(sizeof(qb) / sizeof(qb[0])); ++e) qb[e] = 0;
 #pragma unroll
@@ -834,13 +845,13 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
     const int LA = d.LA, LB = d.LB, padA = d.padA;
     const FastDiv divLA = d.divLA, divLB = d.divLB, divSig = d.divSigmaA;
 #pragma unroll
-    for (int u = 0; u < kRegVec; ++u) {
+    for (int u = 0; u < NA; ++u) {
       const int i = tid + u * kThreads;
-      rA[u] = rB[u] = 0;
+      rA[u] = 0;
       if (!(u & 1)) dA[u >> 1] = 0;
       if (BULK) {
         // the A runs are moved by warp 0's bulk copies
-      } else if (i < nvA && shift) {
+      } else if (kShift && i < nvA && shift) {
         // chunk c of run s: source V * (segA[s] / V + c) past the tile's aligned base, slot
         // s * shiftW + V * c; it covers run elements for lo <= x < hi
         const int s = (int)fdiv((uint32_t)i, d.divCM);
@@ -856,9 +867,13 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
         const int sp = (int)fdiv((uint32_t)p, divSig);
         rA[u] = (int32_t)(gA[s] + (p - s * LA));
         dA[u >> 1] |= ((uint32_t)(p + sp * padA) * (uint32_t)sizeof(TA)) << ((u & 1) * 16);
-        lohi |= (1u | (1u << 4)) << (8 * u);  // x = 0 is in [0, 1)
+        lohi |= NA == kRegVec ? (1u | (1u << 4)) << (8 * u) : 1u << u;  // x = 0 is in [0, 1)
       }
-      const int vi = vec_of(i);
+    }
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+      rB[u] = 0;
+      const int vi = vec_of(tid + u * kThreads);
       if (vi >= 0) {
         const int q = vi * VB;
         const int s = (int)fdiv((uint32_t)q, divLB);
@@ -940,7 +955,7 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
       if constexpr (BETA) {
         if constexpr (REG) {
 #pragma unroll
-          for (int u = 0; u < kRegVec; ++u)
+          for (int u = 0; u < NB; ++u)
             if ((vmask >> u) & 1u) cp_async<VB * sizeof(TB)>(sbB + qb_of(u), Bt + rB[u]);
         } else {
           const int LB = d.LB;
@@ -956,10 +971,17 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
     }
     if constexpr (REG) {
 #pragma unroll
-      for (int u = 0; u < kRegVec; ++u) {
-        const uint32_t f = lohi >> (8 * u);
-        if (x + 1 >= (int)(f & 15u) && x < (int)((f >> 4) & 15u))
-          cp_async<VA * sizeof(TA)>(sb + ((dA[u >> 1] >> ((u & 1) * 16)) & 0xffffu), At + rA[u]);
+      for (int u = 0; u < NA; ++u) {
+        if (u == kRegVec && nvA <= kRegVec * kThreads) break;  // (for all threads alike)
+        bool copy;
+        if constexpr (NA == kRegVec) {
+          const uint32_t f = lohi >> (8 * u);
+          copy = x + 1 >= (int)(f & 15u) && x < (int)((f >> 4) & 15u);
+        } else {
+          copy = (lohi >> u) & 1u;
+        }
+        if (copy) cp_async<VA * sizeof(TA)>(sb + ((dA[u >> 1] >> ((u & 1) * 16)) & 0xffffu), At + rA[u]);
+        static_assert(!BETA || NA == NB, "A and B vectors go in turn");
         if (BETA && ((vmask >> u) & 1u)) cp_async<VB * sizeof(TB)>(sbB + qb_of(u), Bt + rB[u]);
       }
     } else {
@@ -1115,7 +1137,8 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
     if (ti.state == 1) {
       if constexpr (REG) {
 #pragma unroll
-        for (int u = 0; u < kRegVec; ++u) {
+        for (int u = 0; u < NB; ++u) {
+          if (u == kRegVec && nvB <= kRegVec * kThreads) break;  // (for all threads alike)
           if ((vmask >> u) & 1u) {
             uint32_t off[VB];
             reg_pos_of(u, off);

@@ -171,6 +171,9 @@ static int64_t run_len(const std::vector<int>& order, const int64_t* ext, const 
 #define TTCB_TABLE_PATH_COST 1.6
 #endif
 
+// Problems that move at least this many bytes may have tiles of eight 4-byte accesses per thread.
+static constexpr double kWideTileBytes = 64e6;
+
 static void eval_tile(const FusedProblem& f, int EA, int EB, bool beta, const ttcb_tuning& tu, TileCand& c) {
   std::vector<int> aord, bord;
   tile_orders(f, c.ext, aord, bord);
@@ -235,8 +238,12 @@ static void eval_tile(const FusedProblem& f, int EA, int EB, bool beta, const tt
   // narrower accesses cost issue slots (the kernels are close to instruction-bound)
   per_elem += TTCB_NARROW_COST * EA * (16.0 / (c.vecA * EA) - 1.0) / 15.0 * 4.0;
   per_elem += TTCB_NARROW_COST * EB * (16.0 / (c.vecB * EB) - 1.0) / 15.0 * 4.0 * (beta ? 1.5 : 1.0);
-  // the fast kernel keeps at most 4 vectors per thread and phase
-  const bool fast = (c.P / c.vecA <= 1024) && (c.P / c.vecB <= 1024);
+  // the staged kernel's register path, with eight 4-byte accesses per thread for large problems only: small
+  // ones need the tiles to fill the SMs, and the batched kernel keeps four
+  double elems = 1;
+  for (int d = 0; d < f.rank; ++d) elems *= (double)f.n[d];
+  const bool large = elems * (EA + EB * (beta ? 2.0 : 1.0)) >= kWideTileBytes;
+  const bool fast = large ? ttcb::reg_path_fits(c.P, c.vecA, EA, c.vecB, EB, beta) : c.P / c.vecA <= 1024 && c.P / c.vecB <= 1024;
   if (!fast) per_elem *= TTCB_TABLE_PATH_COST;
 
   // average useful elements per tile (ragged last blocks waste a tile's fixed cost)
@@ -911,7 +918,8 @@ static void build_tile_desc(ttcb_plan* p, const TileCand& c, int EA) {
     td.async_ok = (mA < (int64_t(1) << 31) && mB < (int64_t(1) << 31) && td.stage_elems < 65536 &&
                    smem_for(td.nstages) <= 200 * 1024) ? 1 : 0;
     p->smem_async = (int)smem_for(td.nstages);
-    td.reg_ok = (td.fast && td.stage_elems * (int64_t)EA < 65536 && P * (int64_t)EB < 65536) ? 1 : 0;
+    td.reg_ok = (mA < (int64_t(1) << 31) && mB < (int64_t(1) << 31) && ttcb::reg_path_fits(P, c.vecA, EA, c.vecB, EB, beta) &&
+                 td.stage_elems * (int64_t)EA < 65536 && P * (int64_t)EB < 65536) ? 1 : 0;
     // with shifted runs every chunk slot is a copy: the register path holds four per thread (bulk
     // copies of shifted runs hold none)
     if (shift && !bulk && (P / c.LA) * CM > 4 * 256) td.reg_ok = 0;
