@@ -103,7 +103,7 @@ typedef struct {
   int32_t claim_group;   /* staged tile kernel with claimed tiles: consecutive tiles per claim
                             (1..8; more counts as 8); 0 = planner's choice (4 for tiles under
                             13 KiB, 1 for tiles of 20 KiB or more in three stages with B runs
-                            of at most 160 bytes, else 2)                                       */
+                            of at most 160 but not 64 bytes, else 2)                            */
 } ttcb_tuning;
 
 typedef struct ttcb_plan ttcb_plan;

@@ -185,11 +185,12 @@ static ttcb_status plan_finish_device(ttcb_plan* p) {
       // over the sweep, four against two: 0.88-0.99 of the time for tiles of 6-12 KiB, 1.01-1.08 for tiles
       // of 14 KiB and more), else two; but one of tiles of 20 KiB and more in a three-stage ring whose B
       // runs are at most 160 bytes, so that neighbours, which share lines or DRAM bursts of B, are
-      // written by different CTAs at the same time (one against two on 8 such shapes of 200 MiB: 0.88-0.99
-      // of the time; with longer runs or deeper rings 1.00-1.17).
+      // written by different CTAs at the same time (one against two on 10 such shapes of 200 MiB: 0.89-1.01
+      // of the time; with longer runs or deeper rings 1.00-1.17). Of 64-byte runs a pair fills a line:
+      // two again (fp64 with beta, 99.8 against 104.8 us and 91.4 against 100.7).
       const int64_t tile_bytes = td->P * elem_bytes;
-      const bool short_b = tile_bytes >= kClaimSingleTileBytes && td->nstages == 3 &&
-                           td->LB * (int64_t)dtype_bytes(p->tb) <= 160;
+      const int64_t b_run = td->LB * (int64_t)dtype_bytes(p->tb);
+      const bool short_b = tile_bytes >= kClaimSingleTileBytes && td->nstages == 3 && b_run <= 160 && b_run != 64;
       const int group = tile_bytes < kClaimPairTileBytes ? 4 : short_b ? 1 : 2;
       p->claim_group = p->tuning.claim_group > 0 ? std::min(p->tuning.claim_group, ttcb::kDecodeBatch) : group;
       if (p->tuning.round_robin == -1 || claims_by_default) {

@@ -1043,9 +1043,11 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
   // decoded in batches (see TileInfo).
   const int D = S - 2;
   // DYN: tiles 0 .. (D + 2) * G - 1 go round robin (decoded before the previous launch is waited for);
-  // then warp 0 takes claim_group consecutive tiles per claim, issued a group ahead. Lane 0's `pending`
-  // is the first tile of the next group; `cleft` counts the iterations until it is decoded.
+  // then warp 0 takes claim_group consecutive tiles per claim, issued ahead of their decode. Lane 0's
+  // `pending` is the next tile to decode; `cleft` counts the iterations until then.
   unsigned int pending = ntiles, cleft = 0;
+  const unsigned int batch = claim_group == 2 ? 1 : claim_group;
+  bool second = false;  // lane 0: pending is the second tile of a pair
   const unsigned int claim0 = (unsigned int)(D + 2) * G;
   const bool claiming = DYN && claim0 < ntiles;
   uint32_t phase = 0;        // BULK: bit s = parity of the next phase of stage s's barrier
@@ -1111,15 +1113,25 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
       __syncthreads();
     }
     if constexpr (DYN) {
-      // the tiles of iterations k + D + 2 .. k + D + 1 + claim_group, one lane each (the first is read
-      // after the next barrier; the ring entries they replace are of tiles before k), and the next
-      // claim, whose result is needed a group later
+      // Every `batch` iterations warp 0 decodes the tiles of iterations k + D + 2 .. k + D + 1 + batch, one
+      // lane each (the first is read after the next barrier; the ring entries they replace are of tiles
+      // before k), and issues the next claim, whose result is needed at the next decode. The two tiles of
+      // a pair are decoded an iteration apart: together, they made warp 0 late every other iteration (fp64
+      // with beta, 64-byte B runs: 111 us against 102).
       if (cleft == 0) {
-        cleft = claim_group;
+        cleft = batch;
         if (tid < 32) {
           const unsigned int t = __shfl_sync(0xffffffffu, pending, 0) + (unsigned int)tid;
-          if (tid < (int)claim_group) decode_into(t, info[(k + D + 2 + tid) % kInfoRing]);
-          if (claiming && tid == 0) pending = claim0 + atomicAdd(&sched[0], claim_group);
+          if (tid < (int)batch) decode_into(t, info[(k + D + 2 + tid) % kInfoRing]);
+          if (tid == 0) {
+            if (claim_group == 2 && !second) {
+              ++pending;
+              second = true;
+            } else {
+              if (claiming) pending = claim0 + atomicAdd(&sched[0], claim_group);
+              second = false;
+            }
+          }
         }
       }
       --cleft;
