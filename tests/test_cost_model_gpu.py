@@ -88,6 +88,18 @@ def test_whole_network_passes_at_block_edges(rows, nin):
         assert float((got - w).norm()) <= 1e-5 * float(w.norm()), (k, float((got - w).norm()), float(w.norm()))
 
 
+def test_loss_of_an_empty_batch_is_zero():
+    """loss_grad of no rows: a loss of 0 (not what the memory held before) and an empty gradient."""
+    import torch
+    net = _net(5, 128, 0)
+    empty = torch.empty((0, 1), device="cuda")
+    for _ in range(4):
+        stale = [torch.full((1,), 7.0, device="cuda") for _ in range(64)]
+        del stale  # the allocator hands these out again
+        loss, d = net.loss_grad(empty, empty)
+        assert float(loss.item()) == 0.0 and d.shape == (0, 1)
+
+
 def test_gradients_match_torch_autograd_fp32():
     import torch
     net = _net(11, 128, 3)

@@ -304,7 +304,8 @@ class MLP:
     def loss_grad(self, out, y):
         import torch
         d = torch.empty_like(out)
-        loss = torch.empty(1, device="cuda")
+        # (the library writes no loss for an empty batch: 0)
+        loss = (torch.empty if out.numel() else torch.zeros)(1, device="cuda")
         _native.check(_lib().ttcb_mlp_mse(out.data_ptr(), y.data_ptr(), out.numel(), d.data_ptr(), loss.data_ptr(),
                                           _s()))
         return loss, d
