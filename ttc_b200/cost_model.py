@@ -312,9 +312,13 @@ class MLP:
 
     def step(self, grads, lr=1e-3, weight_decay=0.0):
         self.t += 1
-        n = (ctypes.c_int * len(self.params))(*[p.numel() for p in self.params])
-        _native.check(_lib().ttcb_mlp_adam_multi(len(self.params), _ptrs(self.params), _ptrs(grads), _ptrs(self.m),
-                                                 _ptrs(self.v), n, lr, 0.9, 0.999, 1e-8, weight_decay, self.t, _s()))
+        pairs = list(zip(self.params, grads, self.m, self.v))  # as many tensors as there are gradients
+        if not pairs:
+            return
+        params, grads, m, v = zip(*pairs)
+        n = (ctypes.c_int * len(params))(*[p.numel() for p in params])
+        _native.check(_lib().ttcb_mlp_adam_multi(len(params), _ptrs(params), _ptrs(grads), _ptrs(m), _ptrs(v), n, lr,
+                                                 0.9, 0.999, 1e-8, weight_decay, self.t, _s()))
 
     # -- normalisation and I/O ------------------------------------------------------------------
     def _norm(self, X: np.ndarray):
