@@ -54,3 +54,26 @@ def test_invalid_modes_are_rejected():
         plan_contraction("abz", "bc", "ac")  # z in A only
     with pytest.raises(TTCError):
         plan_contraction("ab", "bc", "acy")  # y in C only
+
+
+@pytest.mark.parametrize("a,b,c", PATTERNS)
+@pytest.mark.parametrize("kind", [str, list, tuple])
+def test_contract_takes_any_sequence_of_modes(monkeypatch, a, b, c, kind):
+    """contract() with the modes as strings, lists and tuples, its transpositions replaced by torch's on
+    the host: the same result, numpy.einsum's, on a first call and a repeated one."""
+    import torch
+    from ttc_b200 import ttgt
+
+    def transpose(src, dst, perm, size, alpha, beta, stream):
+        nd = np.transpose(src.numpy().reshape(size, order="F"), perm)
+        dst.copy_(torch.from_numpy(alpha * nd.reshape(-1, order="F") + (beta * dst.numpy() if beta else 0.0)))
+
+    monkeypatch.setattr(ttgt, "_transpose", transpose)
+    rng = np.random.default_rng(len(a + b + c))
+    ext = {m: int(rng.integers(2, 6)) for m in sorted(set(a + b + c))}
+    A, B, C = (torch.from_numpy(rng.standard_normal(math.prod(ext[m] for m in s))) for s in (a, b, c))
+    nd = lambda flat, s: flat.numpy().reshape([ext[m] for m in s], order="F")
+    want = 0.5 * np.einsum(f"{a},{b}->{c}", nd(A, a), nd(B, b)).reshape(-1, order="F") - 1.5 * C.numpy()
+    for _ in range(2):
+        got = ttgt.contract(A, kind(a), B, kind(b), C.clone(), kind(c), ext, 0.5, -1.5)
+        assert np.allclose(got.numpy(), want, rtol=1e-12, atol=1e-12)

@@ -65,6 +65,13 @@ def _contraction(a: str, b: str, c: str) -> dict:
     return dict(p, a_as_is=p["perm_a"] == list(range(len(a))), b_as_is=p["perm_b"] == list(range(len(b))))
 
 
+def _modes(a, b, c) -> dict:
+    """_contraction for any sequences of modes (lists cannot key the cache: planned on each call)."""
+    if type(a) is type(b) is type(c) is str:
+        return _contraction(a, b, c)
+    return _contraction.__wrapped__(a, b, c)
+
+
 def _transpose(src, dst, perm, size, alpha, beta, stream):
     dtype = torch_letter(src)
     key = (tuple(perm), tuple(size), dtype, complex(beta) != 0, src.device.index)
@@ -79,7 +86,7 @@ def contract(A, a: str, B, b: str, C, c: str, extents: dict, alpha=1.0, beta=0.0
     tensors of one dtype (float32, float64, complex64 or complex128), in TTC's column-major layout
     with the extents given per mode. Asynchronous on ``stream`` (default: torch's current stream)."""
     import torch
-    p = _contraction(a, b, c)
+    p = _modes(a, b, c)
     for name, t, s in (("A", A, a), ("B", B, b), ("C", C, c)):
         missing = [m for m in s if m not in extents]
         if missing:
