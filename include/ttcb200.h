@@ -128,9 +128,9 @@ ttcb_status ttcb_plan_create(ttcb_plan** plan, int rank, const int* perm, const 
 ttcb_status ttcb_transpose(const ttcb_plan* plan, const void* A, void* B, const void* alpha,
                            const void* beta, ttcb_stream_t stream);
 /* Calls with one plan may overlap on the GPU (several streams). A plan whose staged kernel claims
- * tiles from counters ("claims" in its description) takes the counter words in turn from 64 slot
- * pairs, so up to 64 of its launches can be in flight at once; a launch captured in a CUDA graph
- * keeps its slot, and replays of that graph must not overlap each other. */
+ * tiles from counters ("claims" in its description) has a pair of counter words for each of the first
+ * 64 streams it is called on; on further streams, and in a CUDA graph, its calls take the round-robin
+ * order instead, so any launches and replays may overlap. */
 
 /* Allocation-free transposition, for callers that may not allocate device memory (their memory is
  * owned by an external pool, or cudaMalloc is forbidden where they run). It has no counterpart in

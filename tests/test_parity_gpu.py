@@ -410,6 +410,60 @@ def test_claimed_tiles_with_concurrent_launches_and_slot_reuse():
     plan.close()
 
 
+def test_claimed_tiles_of_overlapping_launches_have_their_own_counters():
+    """Launches of one plan that run at the same time never share a tile counter, however many launches lie
+    between them: one held back on a stream until 64 launches later, one replayed from a CUDA graph beside
+    a direct one, and one on each of 70 streams; each result bit for bit
+    equal to the oracle's."""
+    import torch
+    from ttc_b200 import Plan
+    perm, size = [2, 0, 1], [67, 45, 311]
+    plan = Plan(perm, size, "s", False, tuning={"blocks": 16, "round_robin": -1, "tile_elems": 256})
+    assert plan.describe()["tile"]["claims"] == 1
+    A, B = make_inputs(size, perm, "s", 300)
+    want = oracle.transpose(A, B, perm, size, 1.5, 0.0, dtype="s")
+    src = torch.from_numpy(A).cuda()
+    dst = [torch.empty_like(src) for _ in range(70)]
+    gate, s1, s2, s3 = (torch.cuda.Stream() for _ in range(4))
+
+    def together(*calls):
+        """Starts the calls at the same time, each on a stream of its own."""
+        for d in dst:
+            d.fill_(float("nan"))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(gate):
+            torch.cuda._sleep(20_000_000)
+            opened = gate.record_event()
+        for st, call in calls:
+            if st is not s3:
+                st.wait_event(opened)
+            with torch.cuda.stream(st):
+                call()
+        torch.cuda.synchronize()
+
+    def check(used, what):
+        for k in used:
+            assert_bitexact(dst[k].cpu().numpy(), want, f"{what}, output {k}")
+
+    between = lambda: [plan(src, dst[2], 1.5, 0.0, s3) for _ in range(63)]
+    for rep in range(4):
+        together((s1, lambda: plan(src, dst[0], 1.5, 0.0, s1)), (s3, between),
+                 (s2, lambda: plan(src, dst[1], 1.5, 0.0, s2)))
+        check((0, 1, 2), "64 launches apart")
+    graphs = []
+    for rep in range(4):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s1):
+            plan(src, dst[0], 1.5, 0.0, s1)
+        graphs.append(g)
+        together((s1, g.replay), (s3, between), (s2, lambda: plan(src, dst[1], 1.5, 0.0, s2)))
+        check((0, 1, 2), "a replay beside a launch")
+    together(*[(torch.cuda.Stream(), lambda k=k: plan(src, dst[k], 1.5, 0.0)) for k in range(70)])
+    check(range(70), "70 streams")
+    del graphs
+    plan.close()
+
+
 SHIFTED = [([1, 0], [99, 1001]), ([1, 0, 3, 2], [99, 17, 35, 3]), ([1, 0, 2], [45, 77, 9]),
            ([2, 1, 0], [10, 25, 2097]), ([0, 2, 1], [31, 110, 15]), ([2, 0, 1], [23, 13, 240])]
 

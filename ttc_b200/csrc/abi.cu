@@ -76,10 +76,30 @@ void allow_large_smem(const void* func) {
 }  // namespace ttcb
 
 namespace ttcb {
-unsigned int* plan_claim_slot(const ttcb_plan* p) {
-  if (!p->claim_words || !p->launch_count) return nullptr;
-  const unsigned int k = static_cast<std::atomic<unsigned int>*>(p->launch_count)->fetch_add(1);
-  return p->claim_words + 2 * (k % kClaimSlots);
+namespace {
+struct ClaimStreams {
+  std::mutex mutex;
+  int n = 0;
+  unsigned long long id[kClaimSlots];
+};
+}  // namespace
+
+unsigned int* plan_claim_slot(const ttcb_plan* p, cudaStream_t stream) {
+  if (!p->claim_words || !p->claim_streams) return nullptr;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+      cudaStreamGetId(stream, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  ClaimStreams& c = *static_cast<ClaimStreams*>(p->claim_streams);
+  std::lock_guard<std::mutex> lk(c.mutex);
+  int k = 0;
+  while (k < c.n && c.id[k] != id) ++k;
+  if (k == kClaimSlots) return nullptr;
+  if (k == c.n) c.id[c.n++] = id;
+  return p->claim_words + 2 * k;
 }
 }  // namespace ttcb
 
@@ -202,8 +222,8 @@ static ttcb_status plan_finish_device(ttcb_plan* p) {
         }
         if ((e = cudaMemset(p->claim_words, 0, sizeof(unsigned int) * 2 * ttcb::kClaimSlots)) != cudaSuccess)
           return cuda_fail(e, "cudaMemset of the tile counters");
-        p->launch_count = new (std::nothrow) std::atomic<unsigned int>(0);
-        if (!p->launch_count) return fail(TTCB_ERR_ALLOC, "host allocation of the launch counter failed");
+        p->claim_streams = new (std::nothrow) ttcb::ClaimStreams;
+        if (!p->claim_streams) return fail(TTCB_ERR_ALLOC, "host allocation of the tile counters' streams failed");
       }
       if (td->bulkA) {
         e = cudaMalloc(&p->wait_status, sizeof(unsigned int));
@@ -422,7 +442,7 @@ void ttcb_plan_destroy(ttcb_plan* plan) {
   if (plan->dev_desc) cudaFree(plan->dev_desc);
   if (plan->claim_words) cudaFree(plan->claim_words);
   if (plan->wait_status) cudaFree(plan->wait_status);
-  delete static_cast<std::atomic<unsigned int>*>(plan->launch_count);
+  delete static_cast<ttcb::ClaimStreams*>(plan->claim_streams);
   if (plan->side_stream) cudaStreamDestroy(static_cast<cudaStream_t>(plan->side_stream));
   if (plan->ev_fork) cudaEventDestroy(static_cast<cudaEvent_t>(plan->ev_fork));
   if (plan->ev_join) cudaEventDestroy(static_cast<cudaEvent_t>(plan->ev_join));

@@ -62,9 +62,13 @@ static cudaError_t launch_async(const ttcb_plan* p, const void* A, void* B, cons
   std::memset(&be, 0, sizeof(TB));
   if (BETA) std::memcpy(&be, beta, sizeof(TB));
   unsigned int* sched = nullptr;
-  if (DYN) {
-    sched = plan_claim_slot(p);
-    if (!sched) return cudaErrorInvalidValue;
+  if constexpr (DYN) {
+    sched = plan_claim_slot(p, stream);
+    if (!sched) {
+      if (needs_large_smem(p->smem_async))
+        allow_large_smem(reinterpret_cast<const void*>(&tile_async_kernel<TA, TB, VA, VB, BETA, STREAM, REG, false, BULK>));
+      return launch_async<VA, VB, BETA, STREAM, REG, false, BULK>(p, A, B, alpha, beta, stream, blocks);
+    }
   }
   // programmatic stream serialization: the kernel may start while the previous one in the stream
   // drains; it waits (griddepcontrol.wait) before it touches A or B

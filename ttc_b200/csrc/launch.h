@@ -19,12 +19,14 @@ struct KernelRef {
 // One definition per A/B type pair lives in kernels_<pair>.cu.
 KernelRef pick_kernel(ttcb_dtype ta, ttcb_dtype tb, int kernel, int va, int vb, int variant);
 
-// The counter words (claim, finished CTAs) of the next launch of a plan's staged kernel with claimed
-// tiles: one of the plan's kClaimSlots slot pairs, taken in turn, so launches of one plan on
-// different streams use different words (up to kClaimSlots of them in flight). Null when the plan
-// has no counters.
+// The counter words (claim, finished CTAs) of a launch of a plan's staged kernel with claimed tiles on
+// `stream`. Two launches that run at the same time must not share them, so each stream (by its id, which
+// the CUDA runtime never gives out twice) has a pair of its own, whose launches follow each other. Null,
+// and the launch takes the round-robin order, when the plan has no counters, when kClaimSlots other
+// streams have taken them, and under capture: a graph may be replayed beside any launch, and more than
+// once at a time.
 constexpr int kClaimSlots = 64;
-unsigned int* plan_claim_slot(const ttcb_plan* p);
+unsigned int* plan_claim_slot(const ttcb_plan* p, cudaStream_t stream);
 
 // Dynamic shared memory ceiling of every plan (the planner never exceeds it).
 constexpr int kMaxDynamicSmem = 200 * 1024;

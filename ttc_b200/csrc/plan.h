@@ -73,10 +73,10 @@ struct ttcb_plan {
   void* ev_join = nullptr;      // cudaEvent_t
   void* fork_mutex = nullptr;   // std::mutex
   // staged kernel with claimed tiles: kClaimSlots pairs of counter words on the device (zeroed at
-  // creation, reset by each launch's last CTA) and the host's running launch count
+  // creation, reset by each launch's last CTA) and the streams they belong to (see plan_claim_slot)
   unsigned int* claim_words = nullptr;
-  int claim_group = 1;           // tiles per claim
-  void* launch_count = nullptr;  // std::atomic<unsigned int>
+  int claim_group = 1;            // tiles per claim
+  void* claim_streams = nullptr;  // ClaimStreams (abi.cu)
   // staged kernel with bulk A copies: count of stage waits that ran out of time (device word, zeroed
   // at creation; read and cleared by ttcb_plan_wait_timeouts)
   unsigned int* wait_status = nullptr;
