@@ -7,6 +7,7 @@ than the <= 1 ulp the contracted reference would allow.
 import numpy as np
 import pytest
 
+import kernel_sim
 import oracle
 from helpers import (assert_bitexact, make_inputs, split, ttc_cases, uniform, NP, buffer_len)
 
@@ -335,6 +336,67 @@ def test_edge_plans_random_ragged_problems(offset):
         desc = check_case(perm, size, dtype, 1.5, beta, lda, ldb, tuning, seed=100 + it, offset=offset)
         with_edges += bool(desc.get("edges"))
     assert with_edges >= 12, with_edges
+
+
+# problems whose ragged tiles are too many for the staged kernel's own launch: one ragged dimension or two
+EDGE_PLANS = [("s", -0.5, [1, 0, 2], [131, 131, 257], 512, 2), ("d", -0.5, [3, 0, 2, 1], [37, 37, 37, 67], 0, 1),
+              ("c", 0.0, [1, 0, 2], [67, 131, 401], 256, 2), ("z", 1.2, [1, 3, 2, 0], [17, 31, 67, 41], 512, 2),
+              ("zc", 0.0, [1, 0, 2], [13, 97, 2053], 0, 1), ("sd", -0.5, [1, 0, 3, 2], [97, 31, 67, 17], 8192, 1)]
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("dtype,beta,perm,size,tile_elems,boxes", EDGE_PLANS)
+def test_edge_plans_on_streams_in_graphs_and_batches(dtype, beta, perm, size, tile_elems, boxes, offset):
+    """Ragged tiles that edge plans move: the plan says that its own launch does not move them, and the
+    result is the oracle's bit for bit on the default stream, on a side stream, replayed from a captured
+    graph and as a problem of a batch, from aligned and misaligned pointers."""
+    torch = _torch()
+    from ttc_b200 import Plan
+    from ttc_b200.batched import Batch
+    A, B = make_inputs(size, perm, dtype, 41)
+    want = oracle.transpose(A, B.copy(), perm, size, 1.5, beta, dtype=dtype)
+    plan = Plan(perm, size, dtype, beta != 0, tuning={"tile_elems": tile_elems})
+    d = plan.describe()
+    assert d["tile"]["ragged_inline"] == 0 and len(d["edges"]) == boxes and all("plan" in e for e in d["edges"]), d
+    dA = torch.from_numpy(np.concatenate([A[:offset], A])).cuda()[offset:]
+    room = torch.empty(offset + B.size + 8, dtype=torch.from_numpy(B).dtype, device="cuda")
+    dB = room[offset:offset + B.size]
+    side = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        plan(dA, dB, 1.5, beta, side)
+    batch = Batch([plan], [dA], [dB], alpha=1.5, beta=beta)
+
+    def on_side():
+        with torch.cuda.stream(side):
+            plan(dA, dB, 1.5, beta, side)
+
+    for what, call in (("default", lambda: plan(dA, dB, 1.5, beta)), ("stream", on_side), ("graph", graph.replay),
+                       ("batch", batch.launch), ("batch graph", lambda: batch.launch(graph=True))):
+        room.fill_(3.0)
+        dB.copy_(torch.from_numpy(B))
+        torch.cuda.synchronize()
+        call()
+        torch.cuda.synchronize()
+        assert_bitexact(dB.cpu().numpy(), want, f"{what} {dtype} {d['tile']}")
+        assert bool((room[offset + B.size:] == 3.0).all()) and bool((room[:offset] == 3.0).all()), what
+    batch.close()
+    del graph
+    plan.close()
+
+
+def test_plans_that_move_ragged_tiles_in_their_own_launch_have_no_edge_plans():
+    """Their description lists the boxes that the ragged tiles cover, without plans; the same boxes that
+    the edge plans of ragged tiles would have."""
+    _torch()
+    from ttc_b200 import Plan
+    for perm, size in [([2, 0, 1], [67, 131, 251]), ([1, 0], [65, 129]), ([2, 0, 1], [67, 31, 53])]:
+        plan = Plan(perm, size, "s", False)
+        d = plan.describe()
+        assert d["tile"]["ragged_inline"] > 0 and d["edges"], d
+        boxes = kernel_sim.edge_boxes(perm, size, "s", False)
+        assert d["edges"] == [{"offA": b["offA"], "offB": b["offB"]} for b in boxes]
+        plan.close()
 
 
 @pytest.mark.parametrize("dtype,beta", [("s", 0.0), ("s", -0.5), ("d", 0.0), ("d", -0.5), ("c", 1.2), ("zc", 0.0),

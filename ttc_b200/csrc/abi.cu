@@ -345,7 +345,8 @@ static ttcb_status launch_plan(const ttcb_plan* p, const void* A, void* B, const
 
 // Edge plans: the boxes of a staged-kernel plan's ragged tiles, each planned as a transposition of
 // its own (default schedule, the caller's streaming choice) so that the staged kernel moves them
-// too. A box that cannot be planned leaves all of them to the element-wise ragged-tile kernel.
+// too. A box that cannot be planned leaves all of them to the element-wise ragged-tile kernel. A plan
+// whose ragged tiles the staged kernel moves in its own launch has no edge plans.
 static void plan_create_edges(ttcb_plan* p) {
   if (p->depth > 0 || p->empty || p->kernel != TTCB_KERNEL_TILE || p->tuning.ragged == 1) return;
   if (p->tuning.tile_variant == 1 || p->tuning.tile_variant == 2) return;  // kernels without ragged split
@@ -365,6 +366,7 @@ static void plan_create_edges(ttcb_plan* p) {
       q->ldb[i] = box[k].ldb[i];
     }
     q->ta = p->ta;
+  if (p->rag_inline) return;
     q->tb = p->tb;
     q->beta_nonzero = p->beta_nonzero;
     q->tuning.streaming = p->tuning.streaming;

@@ -136,7 +136,7 @@ ttcb_status ttcb_batch_create(ttcb_batch** out, int count, const ttcb_plan* cons
       batch_free(b);
       return bfail(TTCB_ERR_INVALID_ARG, "A or B of problem " + std::to_string(i) + " is NULL");
     }
-    const bool edges = !p->empty && p->kernel == TTCB_KERNEL_TILE && p->nedge > 0 && !p->rag_inline;
+    const bool edges = !p->empty && p->kernel == TTCB_KERNEL_TILE && p->nedge > 0;
     ent.push_back({p, A[i], B[i], edges ? 1 : 0, 1});
     for (int k = 0; edges && k < p->nedge; ++k) {
       const ttcb_plan* q = p->edge[k];

@@ -1348,3 +1348,11 @@ std::string plan_describe_json(const ttcb_plan* p) {
   o << "}";
   return o.str();
 }
+  } else if (p->rag_inline && p->depth == 0 && p->tuning.tile_variant != 1 && p->tuning.tile_variant != 2) {
+    // the boxes that the ragged tiles cover, without plans: the staged kernel's launch moves them
+    EdgeBox box[2];
+    const int n = plan_edge_boxes(p, box);
+    if (n > 0) o << ",\"edges\":[";
+    for (int k = 0; k < n; ++k)
+      o << (k ? "," : "") << "{\"offA\":" << box[k].offA << ",\"offB\":" << box[k].offB << "}";
+    if (n > 0) o << "]";
