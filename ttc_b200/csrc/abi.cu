@@ -348,6 +348,7 @@ static ttcb_status launch_plan(const ttcb_plan* p, const void* A, void* B, const
 // too. A box that cannot be planned leaves all of them to the element-wise ragged-tile kernel. A plan
 // whose ragged tiles the staged kernel moves in its own launch has no edge plans.
 static void plan_create_edges(ttcb_plan* p) {
+  if (p->rag_inline) return;
   if (p->depth > 0 || p->empty || p->kernel != TTCB_KERNEL_TILE || p->tuning.ragged == 1) return;
   if (p->tuning.tile_variant == 1 || p->tuning.tile_variant == 2) return;  // kernels without ragged split
   const TileDesc* td = reinterpret_cast<const TileDesc*>(p->host_desc.data());
@@ -366,7 +367,6 @@ static void plan_create_edges(ttcb_plan* p) {
       q->ldb[i] = box[k].ldb[i];
     }
     q->ta = p->ta;
-  if (p->rag_inline) return;
     q->tb = p->tb;
     q->beta_nonzero = p->beta_nonzero;
     q->tuning.streaming = p->tuning.streaming;

@@ -1344,10 +1344,6 @@ std::string plan_describe_json(const ttcb_plan* p) {
       o << (k ? "," : "") << "{\"offA\":" << p->edge[k]->base_offA << ",\"offB\":" << p->edge[k]->base_offB
         << ",\"plan\":" << plan_describe_json(p->edge[k]) << "}";
     o << "]";
-  }
-  o << "}";
-  return o.str();
-}
   } else if (p->rag_inline && p->depth == 0 && p->tuning.tile_variant != 1 && p->tuning.tile_variant != 2) {
     // the boxes that the ragged tiles cover, without plans: the staged kernel's launch moves them
     EdgeBox box[2];
@@ -1356,3 +1352,7 @@ std::string plan_describe_json(const ttcb_plan* p) {
     for (int k = 0; k < n; ++k)
       o << (k ? "," : "") << "{\"offA\":" << box[k].offA << ",\"offB\":" << box[k].offB << "}";
     if (n > 0) o << "]";
+  }
+  o << "}";
+  return o.str();
+}
