@@ -176,8 +176,9 @@ void ttcb_version(int* major, int* minor, int* patch);
 /* ---------------------------------------------------------------------------------------------
  * Batched mode: many independent transpositions in one persistent launch.
  * No counterpart in TTC, which can only call one generated wrapper per transposition (each with its
- * own cudaMalloc/cudaMemcpy/cudaDeviceSynchronize, CUDAtranspose.py:395-429). The batch owns a
- * device table of per-problem descriptors, a prefix sum of tile counts and a work counter.
+ * own cudaMalloc/cudaMemcpy/cudaDeviceSynchronize, CUDAtranspose.py:395-429). The batch owns the
+ * problems' descriptors, a device table of segments (runs of one problem's tiles or rows), and the counters
+ * from which CTAs claim them. Its launches must follow one another (they write the same B).
  * ------------------------------------------------------------------------------------------- */
 typedef struct ttcb_batch ttcb_batch;
 
@@ -193,7 +194,9 @@ ttcb_status ttcb_batch_launch(ttcb_batch* batch, ttcb_stream_t stream);
 /* Captures the batch launch into a CUDA graph once and replays it. */
 ttcb_status ttcb_batch_graph_launch(ttcb_batch* batch, ttcb_stream_t stream);
 
-/* Device status word of the last launch: 0 = ok, otherwise a TTCB_ERR_* code set on the device. */
+/* Device status word: 0 = ok, otherwise the first TTCB_ERR_* code that a launch of the batch set on the device
+ * (TTCB_ERR_INVALID_ARG: a segment's record was not sound, and the segment was left out). Waits for the
+ * stream, so errors of the launch itself appear here too. */
 ttcb_status ttcb_batch_status(ttcb_batch* batch, ttcb_stream_t stream);
 
 int64_t ttcb_batch_bytes(const ttcb_batch* batch);

@@ -148,6 +148,40 @@ def test_batched_segments(dtype, beta, blocks):
     batch.close()
 
 
+@pytest.mark.parametrize("what,change", [("an unknown kind", (9, -1, -1)), ("no tiles", (-1, 0, -1)),
+                                         ("more tiles than a segment holds", (1, 1000, -1)),
+                                         ("more stages than the ring", (1, -1, 100)), ("no stage", (1, -1, 0))])
+def test_unsound_segments_are_reported_and_left_out(what, change):
+    """A segment record that the kernel cannot work from sets the batch's status word; its problem's B stays
+    as it was, every other problem's is the oracle's, and the counters are sound for the next launch."""
+    import torch
+    from ttc_b200 import Plan, TTCError
+    from ttc_b200._native import lib
+    from ttc_b200.batched import Batch
+    shapes = [([1, 0], [64, 48]), ([2, 1, 0], [8, 16, 32]), ([1, 0], [96, 32])]  # complete tiles, one segment each
+    As = [torch.from_numpy(uniform(int(np.prod(s)), "s", k)).cuda() for k, (_, s) in enumerate(shapes)]
+    Bs = [torch.full_like(a, 5.0) for a in As]
+    batch = Batch([Plan(p, s, "s", False) for p, s in shapes], As, Bs, alpha=1.5, blocks=2)
+    batch.launch()
+    batch.check_status()
+    assert lib().ttcb_test_batch_segment(batch._h, 0, *change) == 1
+    for _ in range(2):
+        for b in Bs:
+            b.fill_(5.0)
+        batch.launch()
+        with pytest.raises(TTCError):
+            batch.check_status()
+        left = 0
+        for a, b, (perm, size) in zip(As, Bs, shapes):
+            got = b.cpu().numpy()
+            if (got == 5.0).all():
+                left += 1
+            else:
+                assert_bitexact(got, oracle.transpose(a.cpu().numpy(), got.copy(), perm, size, 1.5, 0.0, dtype="s"), what)
+        assert left == 1, what
+    batch.close()
+
+
 def test_batch_rejects_mixed_types():
     from ttc_b200 import Plan, TTCError
     from ttc_b200.batched import Batch

@@ -118,6 +118,7 @@ TEST_SYMBOLS = [
     ("ttcb_test_fuse", ctypes.c_int, [ctypes.c_int, _IP, _I64P, _I64P, _I64P, _IP, _IP, _I64P, _I64P, _I64P]),
     ("ttcb_test_plan_host", ctypes.c_int, [ctypes.c_int, _IP, _I64P, _I64P, _I64P, ctypes.c_int, ctypes.c_int,
                                            ctypes.c_int, ctypes.POINTER(Tuning), ctypes.c_char_p, ctypes.c_size_t]),
+    ("ttcb_test_batch_segment", ctypes.c_int, [_P, ctypes.c_uint, ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     ("ttcb_test_plan_desc", ctypes.c_size_t, [_P, _P, ctypes.c_size_t]),
     ("ttcb_test_fastdiv", ctypes.c_uint32, [ctypes.c_uint32, ctypes.c_uint32]),
     ("ttcb_test_plan_host_desc", ctypes.c_size_t, [ctypes.c_int, _IP, _I64P, _I64P, _I64P, ctypes.c_int, ctypes.c_int,

@@ -5,6 +5,7 @@
 // of row units (one per warp) of one problem. A CTA takes two segments round robin and then claims them
 // from a counter, so long and short problems balance across the GPU. Nothing waits on another CTA.
 #pragma once
+#include "../../include/ttcb200.h"
 #include "kernels.cuh"
 
 namespace ttcb {
@@ -36,6 +37,18 @@ struct BatchSeg {
   } g[TTCB_MAXR];
 };
 static_assert(sizeof(BatchSeg) % 16 == 0, "records are copied by 16 bytes");
+
+// Batch status codes written by the device (0 = ok): a TTCB_ERR_* code.
+enum { kBatchBadSegment = TTCB_ERR_INVALID_ARG };
+
+// Whether a segment's record is one that batch_kernel knows, within `smem` bytes of dynamic shared memory.
+__device__ __forceinline__ bool segment_ok(const BatchSeg& s, uint32_t smem) {
+  if (s.nt < 1) return false;
+  if (s.kind == kSegFull)
+    return s.nt <= kSegTiles && s.stages >= 1 && s.stages <= kMaxStages && s.stage_bytes > 0 &&
+           (uint64_t)s.stages * (uint32_t)s.stage_bytes <= smem;
+  return s.kind == kSegRows || (s.kind == kSegRagged && s.stage_bytes > 0 && (uint32_t)s.stage_bytes <= smem);
+}
 
 // CTAs per SM that the register budget is sized for: 4 (64 registers), or 3 when B is read back too, as
 // the staged kernel's. What bounds a batch is latency: a segment starts with its tables and its first copies
@@ -222,7 +235,8 @@ __device__ __noinline__ void batch_rows(const BatchSeg& s, TA alpha, TB beta) {
   }
 }
 
-// counter[0]: segments claimed, counter[1]: finished CTAs; the last one sets both back to zero. CTA b
+// counter[0]: segments claimed, counter[1]: finished CTAs; the last one sets both back to zero.
+// counter[2]: the first error; a segment whose record is not a sound one is left out. CTA b
 // takes segments b and b + gridDim.x first; each further claim is issued two segments ahead and each record
 // copied one ahead, so neither is waited for.
 template <typename TA, typename TB, bool BETA, bool STREAM>
@@ -262,7 +276,10 @@ __global__ void __launch_bounds__(kThreads, batch_min_blocks(BETA))
       if (n < nseg && tid < kRec16)
         cp_async<16>(smem_u32(&rec[cur ^ 1]) + tid * 16, reinterpret_cast<const unsigned char*>(segs + n) + tid * 16);
     };
-    if (s.kind == kSegFull) {
+    uint32_t smem;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(smem));
+    const bool ok = segment_ok(s, smem);
+    if (ok && s.kind == kSegFull) {
       if (tid < s.nt) {
         uint32_t t = s.t0 + (uint32_t)tid;
         int64_t bA = 0, bB = 0;
@@ -295,7 +312,9 @@ __global__ void __launch_bounds__(kThreads, batch_min_blocks(BETA))
     } else {
       __syncthreads();
       prefetch();
-      if (s.kind == kSegRows)
+      if (!ok) {
+        if (tid == 0) atomicCAS(&counter[2], 0u, (unsigned int)kBatchBadSegment);
+      } else if (s.kind == kSegRows)
         batch_rows<TA, TB, BETA, STREAM>(s, alpha, beta);
       else
         batch_ragged<TA, TB, BETA, STREAM>(s, alpha, beta, d, rag, smem_raw);

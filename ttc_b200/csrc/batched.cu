@@ -398,6 +398,19 @@ ttcb_status ttcb_batch_status(ttcb_batch* b, ttcb_stream_t stream) {
   return TTCB_OK;
 }
 
+int ttcb_test_batch_segment(ttcb_batch* b, unsigned int k, int kind, int nt, int stages) {
+  if (!b || k >= b->nseg) return -1;
+  ttcb::BatchSeg s;
+  unsigned char* at = static_cast<unsigned char*>(b->d_segs) + sizeof(s) * k;
+  if (cudaMemcpy(&s, at, sizeof(s), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
+  const int was = s.kind;
+  if (kind >= 0) s.kind = kind;
+  if (nt >= 0) s.nt = nt;
+  if (stages >= 0) s.stages = stages;
+  if (cudaMemcpy(at, &s, sizeof(s), cudaMemcpyHostToDevice) != cudaSuccess) return -1;
+  return was;
+}
+
 int64_t ttcb_batch_bytes(const ttcb_batch* b) { return b ? b->bytes : 0; }
 
 void ttcb_batch_destroy(ttcb_batch* b) { batch_free(b); }

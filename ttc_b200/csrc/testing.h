@@ -1,5 +1,5 @@
 // Test hooks exported by libttcb200.so for unit tests. They are not part of the public ABI
-// (include/ttcb200.h); all but ttcb_test_bounded_wait make no CUDA calls.
+// (include/ttcb200.h); all but ttcb_test_bounded_wait and ttcb_test_batch_segment make no CUDA calls.
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -35,4 +35,7 @@ size_t ttcb_test_plan_edges(int rank, const int* perm, const int64_t* size, cons
 // the phase, so the wait must give up; with arrive = 1 the CTA arrives first, so it must not. Writes
 // to *gave_up how many CTAs gave up (0 or 1); returns the CUDA error code.
 int ttcb_test_bounded_wait(uint64_t limit_ns, int arrive, unsigned int* gave_up);
+// Overwrites fields of a batch's k-th segment record on the device (negative: as it is) with values that
+// batch_kernel has to recognise as unsound. Returns the record's kind before, -1 on failure.
+int ttcb_test_batch_segment(ttcb_batch* batch, unsigned int k, int kind, int nt, int stages);
 }
