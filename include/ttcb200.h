@@ -101,7 +101,7 @@ typedef struct {
                             planner's model finds fewer bank conflicts in the gather that way;
                             0 or -1 = a warp takes 32 consecutive B vectors                     */
   int32_t claim_group;   /* staged tile kernel with claimed tiles: consecutive tiles per claim
-                            (1..8; more counts as 8); 0 = planner's choice (4 for tiles under
+                            (1..64; more counts as 64); 0 = planner's choice (4 for tiles under
                             13 KiB, 1 for tiles of 20 KiB or more in three stages with B runs
                             of at most 160 but not 64 bytes, else 2)                            */
 } ttcb_tuning;

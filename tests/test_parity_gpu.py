@@ -472,6 +472,19 @@ def test_claimed_tiles_with_concurrent_launches_and_slot_reuse():
     plan.close()
 
 
+@pytest.mark.parametrize("group", [7, 8, 9, 12, 13, 16, 63, 64, 100])
+def test_claims_of_any_group_size(group):
+    """Claims of up to 64 consecutive tiles (more count as 64), decoded in batches of the largest divisor up to
+    eight: bit for bit against the oracle with few CTAs, which then claim many groups, and many, for the
+    shallowest and the deepest ring, by plain and by bulk copies."""
+    for blocks in (3, 0):
+        for tuning in ({"stages": 3}, {"stages": 7}, {"bulk_copies": 1}):
+            for size in ([67, 45, 311], [64, 48, 16]):
+                desc = check_case([2, 0, 1], size, "s", 1.5, -0.5,
+                                  tuning=dict(tuning, claim_group=group, round_robin=-1, blocks=blocks, tile_elems=256))
+                assert desc["tile"]["claims"] == 1 and desc["tile"]["claim_group"] == min(group, 64), desc
+
+
 def test_claimed_tiles_of_overlapping_launches_have_their_own_counters():
     """Launches of one plan that run at the same time never share a tile counter, however many launches lie
     between them: one held back on a stream until 64 launches later, one replayed from a CUDA graph beside

@@ -212,7 +212,7 @@ static ttcb_status plan_finish_device(ttcb_plan* p) {
       const int64_t b_run = td->LB * (int64_t)dtype_bytes(p->tb);
       const bool short_b = tile_bytes >= kClaimSingleTileBytes && td->nstages == 3 && b_run <= 160 && b_run != 64;
       const int group = tile_bytes < kClaimPairTileBytes ? 4 : short_b ? 1 : 2;
-      p->claim_group = p->tuning.claim_group > 0 ? std::min(p->tuning.claim_group, ttcb::kDecodeBatch) : group;
+      p->claim_group = p->tuning.claim_group > 0 ? std::min(p->tuning.claim_group, ttcb::kMaxClaimGroup) : group;
       if (p->tuning.round_robin == -1 || claims_by_default) {
         e = cudaMalloc(&p->claim_words, sizeof(unsigned int) * 2 * ttcb::kClaimSlots);
         if (e != cudaSuccess) {

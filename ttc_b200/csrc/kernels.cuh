@@ -564,13 +564,23 @@ struct TileInfo {
 
 // Static shared memory of the staged kernel (descriptor header + tile ring), on top of its dynamic
 // shared memory.
-constexpr int kDecodeBatch = 8;              // staged kernel: tiles decoded per batch (and at most per claim)
+constexpr int kDecodeBatch = 8;              // staged kernel: tiles decoded per batch
 constexpr int kInfoRing = 2 * kDecodeBatch;  // decoded-tile ring entries (tile j in entry j % kInfoRing)
 constexpr int kMaxStages = 7;                // S - 2 = D tiles in flight, D < kDecodeBatch
 static_assert(kMaxStages - 2 + kDecodeBatch + 2 <= kInfoRing, "claimed tiles must replace finished ones only");
 static_assert(kMaxStages - 2 < kDecodeBatch && kMaxStages - 2 <= 5,
               "tiles in flight must be decoded a batch ahead and covered by the copy-group wait");
 constexpr size_t kAsyncStaticSmem = sizeof(TileDesc) + kInfoRing * sizeof(TileInfo) + kMaxStages * sizeof(uint64_t);
+
+// Tiles of a claimed group that are decoded at once: a divisor of the group's size, at most kDecodeBatch. A
+// pair is decoded one tile an iteration: together, its tiles made warp 0 late every other iteration (fp64
+// with beta, 64-byte B runs: 111 us against 102).
+constexpr int kMaxClaimGroup = 64;
+__host__ __device__ constexpr int claim_batch(int group) {
+  int b = group < kDecodeBatch ? group : kDecodeBatch;
+  while (group % b != 0) --b;
+  return group == 2 ? 1 : b;
+}
 
 // Tile index of the r-th ragged tile (see TileDesc::rag_a): mixed radix over the grid dimensions
 // with the ragged dimension pinned to its last block (and, in the second part, rag_a below its last).
@@ -726,11 +736,12 @@ __device__ __noinline__ void ragged_pass(const TileDesc& d, const unsigned char*
 // per vector from the run tables in shared memory, with the gather positions in registers while
 // P <= kRegPos * kThreads and in shared memory beyond. The number of stages (3 to kMaxStages) is the
 // descriptor's.
-// DYN: after the first D + 2 tiles of each CTA (round robin), tiles are claimed in order from a counter
+// DYN: after the first D + 2 tiles of each CTA (consecutive), tiles are claimed in order from a counter
 // in global memory (sched[0]) as the CTA goes, instead of the fixed round-robin first + k * gridDim.x.
 // CTAs then stay on neighbouring tiles however their speeds differ, so the tiles in motion stay within
-// a narrow span of A and B, and the last tiles go to whichever CTAs are free. Each claim takes
-// claim_group (1..8) consecutive tiles, decoded by as many lanes at once. The last CTA to finish
+// a narrow span of A and B, and the last tiles go to whichever CTAs are free. Each claim takes a group of
+// consecutive tiles (`claims`: the group's size and, in the upper half, claim_batch of it), decoded by as
+// many lanes at once as a batch has tiles. The last CTA to finish
 // (sched[1] counts them) sets both words back to zero for the next launch that uses them, which runs
 // after this grid completes (stream order, and griddepcontrol.wait before the first claim when the
 // launch overlaps its predecessor). A launch of at most (D + 2) * gridDim.x tiles claims none.
@@ -744,7 +755,7 @@ template <typename TA, typename TB, int VA, int VB, bool BETA, bool STREAM, bool
 __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB * sizeof(TB), BETA))
     tile_async_kernel(
     const TileDesc* __restrict__ desc, const TA* __restrict__ A, TB* __restrict__ B, TA alpha, TB beta,
-    unsigned int* __restrict__ sched, int a0, unsigned int* __restrict__ wait_status, unsigned int claim_group,
+    unsigned int* __restrict__ sched, int a0, unsigned int* __restrict__ wait_status, unsigned int claims,
     int rag) {
   static_assert(!BULK || VA * sizeof(TA) == 16, "bulk copies move runs of whole 16-byte vectors");
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1042,12 +1053,13 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
   // (k - 2) every thread finished writing out before the barrier of iteration k - 1. Tiles are
   // decoded in batches (see TileInfo).
   const int D = S - 2;
-  // DYN: tiles 0 .. (D + 2) * G - 1 go round robin (decoded before the previous launch is waited for);
-  // then warp 0 takes claim_group consecutive tiles per claim, issued ahead of their decode. Lane 0's
-  // `pending` is the next tile to decode; `cleft` counts the iterations until then.
-  unsigned int pending = ntiles, cleft = 0;
-  const unsigned int batch = claim_group == 2 ? 1 : claim_group;
-  bool second = false;  // lane 0: pending is the second tile of a pair
+  // DYN: each CTA starts on D + 2 consecutive tiles (tiles 0 .. (D + 2) * G - 1 in all, decoded before the
+  // previous launch is waited for; a launch that claims none goes round robin); then warp 0 takes
+  // `group` consecutive tiles per claim, issued ahead of their decode, and decodes `batch` of them at a
+  // time. Lane 0's `pending` is the next tile to decode and `left` how many of its claim are left; `cleft`
+  // counts the iterations until then.
+  const unsigned int group = claims & 0xffffu, batch = claims >> 16;
+  unsigned int pending = ntiles, left = group, cleft = 0;
   const unsigned int claim0 = (unsigned int)(D + 2) * G;
   const bool claiming = DYN && claim0 < ntiles;
   uint32_t phase = 0;        // BULK: bit s = parity of the next phase of stage s's barrier
@@ -1066,7 +1078,7 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
   // everything above reads the plan's descriptor only; A and B are touched from here on
   pdl_wait_previous();
   // (the previous launch's reset of the counter is visible from here)
-  if (claiming && tid == 0) pending = claim0 + atomicAdd(&sched[0], claim_group);
+  if (claiming && tid == 0) pending = claim0 + atomicAdd(&sched[0], group);
   for (int j = 0; j < D; ++j) {
     issue(info[j], j);
     cp_async_commit();
@@ -1115,21 +1127,20 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
     if constexpr (DYN) {
       // Every `batch` iterations warp 0 decodes the tiles of iterations k + D + 2 .. k + D + 1 + batch, one
       // lane each (the first is read after the next barrier; the ring entries they replace are of tiles
-      // before k), and issues the next claim, whose result is needed at the next decode. The two tiles of
-      // a pair are decoded an iteration apart: together, they made warp 0 late every other iteration (fp64
-      // with beta, 64-byte B runs: 111 us against 102).
+      // before k), and after a group's last batch issues the next claim, whose result is needed at the
+      // next decode.
       if (cleft == 0) {
         cleft = batch;
         if (tid < 32) {
           const unsigned int t = __shfl_sync(0xffffffffu, pending, 0) + (unsigned int)tid;
           if (tid < (int)batch) decode_into(t, info[(k + D + 2 + tid) % kInfoRing]);
           if (tid == 0) {
-            if (claim_group == 2 && !second) {
-              ++pending;
-              second = true;
+            left -= batch;
+            if (left != 0) {
+              pending += batch;
             } else {
-              if (claiming) pending = claim0 + atomicAdd(&sched[0], claim_group);
-              second = false;
+              left = group;
+              if (claiming) pending = claim0 + atomicAdd(&sched[0], group);
             }
           }
         }
