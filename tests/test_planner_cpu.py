@@ -474,6 +474,20 @@ def test_lane_maps():
     assert maps >= 10 and sorted_runs >= 2, (maps, sorted_runs)
 
 
+@pytest.mark.parametrize("perm,size,vec,ragged,wide", [
+    ([2, 0, 3, 1], [1254, 22, 2, 305], (2, 4), 0, False), ([1, 0, 2], [65, 17, 12981], (2, 2), 1, False),
+    ([2, 1, 4, 0, 3], [897, 2, 7, 104, 17], (1, 2), 0, False), ([1, 3, 5, 2, 4, 0], [10, 31, 11, 99, 2, 78], (2, 1), 0, False),
+    ([1, 0], [27, 1941807], (4, 1), 1, True), ([2, 1, 0], [10, 25, 209715], (2, 1), 0, True)])
+def test_tiles_of_eight_accesses_keep_access_widths_and_ragged_tiles(perm, size, vec, ragged, wide):
+    """A tile of more than four 4-byte accesses per thread is taken (fp32, beta = 0, 64 MB and more) only where
+    the accesses are as wide as those of the tile that would be taken without them, and the ragged tiles as
+    few."""
+    j = plan_host_json(perm, size, "s", False)
+    t = j["tile"]
+    assert j["vecA"] >= vec[0] and j["vecB"] >= vec[1] and t["ragged_tiles"] <= ragged, j
+    assert (t["reg"] == 1 and max(t["P"] // j["vecA"], t["P"] // j["vecB"]) > 1024) == wide, j
+
+
 def test_ragged_tiles_moved_by_vectors_have_whole_vectors():
     """When the staged kernel moves ragged tiles by vectors (ragged_inline 1), every vector of a ragged
     tile is valid as a whole or not at all, in A order (vecA) and in B order (vecB), and at aligned
