@@ -433,9 +433,10 @@ __global__ void __launch_bounds__(kThreads, 3) tile_fast_kernel(const TileDesc* 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // Programmatic dependent launch: a kernel launched with programmatic stream serialization may start
-// while the kernel before it in the stream drains. It lets its own successor start early as soon as
-// every CTA has begun (launch_dependents), and it touches no tensor data before everything the
-// previous kernel wrote is visible (wait). Both are no-ops in a launch without the attribute.
+// while the kernel before it in the stream drains, and touches no tensor data before everything the
+// previous kernel wrote is visible (wait). A launch may let its own successor start as soon as every CTA of
+// it has begun (launch_dependents); else the successor starts when every CTA has ended. Both are no-ops in
+// a launch without the attribute.
 __device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
@@ -608,14 +609,15 @@ __device__ __forceinline__ uint32_t ragged_tile_index(const TileDesc& d, uint32_
   return t;
 }
 
-// Ragged tiles inside the staged kernel (kernel argument `rag`): CTA b moves ragged tiles b, b + G, ..
+// Ragged tiles inside the staged kernel (kRagMask of its argument `flags`): CTA b moves ragged tiles b, b + G, ..
 // before its complete tiles, through two stages of its ring. A launch of its own for them costs a fork
 // to a side stream and a join back: about 4 us on the device, where the call after it can then not
 // start while this one drains, and 5.5 us on the host. Elements go V at a time when every tile limit falls
 // on a multiple of V in both orders (kRagVec: V is the access width), else one at a time. The pass is
 // a call of its own, ahead of the ring's set-up, so that the ring keeps its registers (with the ragged
 // tiles in the ring's own order, scalar fp32 instantiations spilled and ran 4-9% slower).
-enum { kRagNone = 0, kRagVec = 1, kRagScalar = 2 };
+enum { kRagNone = 0, kRagVec = 1, kRagScalar = 2, kRagMask = 3 };
+constexpr int kOverlapNext = 4;  // flags: let the next launch of the stream begin beside this one (see abi.cu)
 
 // Whether A-order (B-order: tsB) position p lies within the tile's limits.
 template <bool ORDER_B>
@@ -756,14 +758,15 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
     tile_async_kernel(
     const TileDesc* __restrict__ desc, const TA* __restrict__ A, TB* __restrict__ B, TA alpha, TB beta,
     unsigned int* __restrict__ sched, int a0, unsigned int* __restrict__ wait_status, unsigned int claims,
-    int rag) {
+    int flags) {
   static_assert(!BULK || VA * sizeof(TA) == 16, "bulk copies move runs of whole 16-byte vectors");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ TileDesc d;  // the descriptor header, read once per CTA
   __shared__ TileInfo info[kInfoRing];  // kAsyncStaticSmem counts both, and the stage barriers
   __shared__ __align__(8) uint64_t abar[kMaxStages];  // BULK: one mbarrier per stage
   const int tid = threadIdx.x;
-  pdl_allow_next();
+  const int rag = flags & kRagMask;
+  if (flags & kOverlapNext) pdl_allow_next();
   for (int i = tid; i < (int)(sizeof(TileDesc) / 4); i += kThreads)
     reinterpret_cast<uint32_t*>(&d)[i] = reinterpret_cast<const uint32_t*>(desc)[i];
   __syncthreads();

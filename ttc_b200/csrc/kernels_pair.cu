@@ -87,7 +87,8 @@ static cudaError_t launch_async(const ttcb_plan* p, const void* A, void* B, cons
   return cudaLaunchKernelEx(&cfg, tile_async_kernel<TA, TB, VA, VB, BETA, STREAM, REG, DYN, BULK>,
                             reinterpret_cast<const TileDesc*>(p->dev_desc), static_cast<const TA*>(A),
                             static_cast<TB*>(B), al, be, sched, a0, BULK ? p->wait_status : nullptr,
-                            (unsigned int)(p->claim_group | claim_batch(p->claim_group) << 16), p->rag_inline);
+                            (unsigned int)(p->claim_group | claim_batch(p->claim_group) << 16),
+                            p->rag_inline | (plan_overlaps_next(p, stream) ? kOverlapNext : 0));
 }
 
 template <int VA, int VB, bool REG, bool DYN, bool BULK>

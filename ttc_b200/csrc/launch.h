@@ -28,6 +28,9 @@ KernelRef pick_kernel(ttcb_dtype ta, ttcb_dtype tb, int kernel, int va, int vb, 
 constexpr int kClaimSlots = 64;
 unsigned int* plan_claim_slot(const ttcb_plan* p, cudaStream_t stream);
 
+// Whether a launch of the staged kernel lets its successor in the stream begin beside it (abi.cu: the reason).
+bool plan_overlaps_next(const ttcb_plan* p, cudaStream_t stream);
+
 // Dynamic shared memory ceiling of every plan (the planner never exceeds it).
 constexpr int kMaxDynamicSmem = 200 * 1024;
 // True when a launch with this much dynamic shared memory needs the opt-in above 48 KB.
