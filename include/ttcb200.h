@@ -85,8 +85,9 @@ typedef struct {
                             copies in flight); 0 = planner's choice                             */
   int32_t ctas_per_sm;   /* staged tile kernel: resident CTAs per SM (1..8, capped by what fits);
                             0 = planner's choice. `blocks`, when set, takes precedence          */
-  int32_t round_robin;   /* staged tile kernel: 0 = planner's choice (claims for calls that move
-                            128 MB or more, 150 MB with beta, with 8 or more tiles per CTA), 1 = fixed round-robin order
+  int32_t round_robin;   /* staged tile kernel: 0 = planner's choice (claims for tensors of
+                            160 MB or more with 8 or more tiles per CTA, but for small tiles with long
+                            runs on both sides and thin matrices with beta), 1 = fixed round-robin order
                             (tile blockIdx + k * CTAs), -1 = CTAs claim tiles in order from
                             counters the plan owns                                              */
   int32_t shifted_runs;  /* staged tile kernel: 1 = copy A runs that 16-byte accesses cannot
@@ -102,8 +103,7 @@ typedef struct {
                             0 or -1 = a warp takes 32 consecutive B vectors                     */
   int32_t claim_group;   /* staged tile kernel with claimed tiles: consecutive tiles per claim
                             (1..64; more counts as 64); 0 = planner's choice (4 for tiles under
-                            13 KiB, 1 for tiles of 20 KiB or more in three stages with B runs
-                            of at most 160 but not 64 bytes, else 2)                            */
+                            13 KiB, else 2)                                                     */
 } ttcb_tuning;
 
 typedef struct ttcb_plan ttcb_plan;

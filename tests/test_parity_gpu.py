@@ -472,6 +472,63 @@ def test_claimed_tiles_with_concurrent_launches_and_slot_reuse():
     plan.close()
 
 
+def test_large_plans_in_turn_and_in_a_row_see_each_others_results():
+    """Launches of different and of the same plans behind each other on one stream, each reading what the one
+    before wrote, below and above the size from which a launch lets the next one begin beside it only when
+    it repeats its plan: bit for bit torch's permutations."""
+    torch = _torch()
+    from ttc_b200 import Plan
+
+    def permuted(t, perm):  # t: row-major view of the column-major tensor
+        n = t.dim()
+        return t.permute(*[n - 1 - perm[j] for j in reversed(range(n))]).contiguous()
+
+    steps = [[2, 0, 1], [2, 0, 1], [1, 0, 2]]
+    for mb in (40, 130):
+        size = [96, 160, mb * 1_000_000 // 8 // (96 * 160)]
+        x = torch.rand(*reversed(size), device="cuda")
+        wants, plans = [x], []
+        for perm in steps:
+            plans.append(Plan(perm, list(reversed(wants[-1].shape)), "s", False))
+            wants.append(permuted(wants[-1], perm))
+        outs = [x] + [torch.empty_like(x) for _ in steps]
+        for repeat in (1, 1, 3, 2, 1):
+            for y in outs[1:]:
+                y.fill_(float("nan"))
+            for p, src, dst in zip(plans, outs, outs[1:]):
+                for _ in range(repeat):
+                    p(src, dst)
+            torch.cuda.synchronize()
+            for k, (y, w) in enumerate(zip(outs[1:], wants[1:])):
+                assert torch.equal(y.view(-1), w.view(-1)), (mb, repeat, k)
+        for p in plans:
+            p.close()
+
+
+@pytest.mark.parametrize("perm,size,dtype,beta,claims,group", [
+    ([1, 0, 2], [1000, 768, 16], "s", 1.0, 0, 2),            # 98 MB of tensors
+    ([1, 0, 2], [1024, 768, 25], "s", 0.0, 0, 2),            # 157 MB
+    ([1, 0, 2], [1024, 768, 26], "s", 0.0, 1, 2),            # 164 MB
+    ([1, 0], [27, 1941807], "s", -0.5, 0, 4),                # thin, with beta: A by 16 bytes, B by 4
+    ([2, 0, 1], [13, 2016492, 2], "s", -0.5, 0, 4),          # tiles of 12 KiB, runs of 2 and 4 KB
+    ([1, 0], [7489829, 7], "s", 0.0, 1, 2),                  # of 14 KiB, runs of 1 and 7 KB, A by 4 bytes
+    ([1, 0, 2], [1565, 1155, 29], "s", -0.5, 1, 4),          # of 12 KiB, runs of 128 bytes
+    ([5, 2, 1, 3, 0, 4], [10, 7, 13, 11, 81, 65], "s", 0.0, 1, 4),  # of 7 KiB, runs of 280 and 52 bytes
+    ([5, 4, 0, 2, 1, 3], [7, 11, 16, 38, 5, 112], "d", -0.5, 1, 2)])  # of 29 KB
+def test_planners_claim_rule(perm, size, dtype, beta, claims, group):
+    """Tiles are claimed by default for tensors past L2, by twos or, of tiles under 13 KiB, by fours, but not small
+    tiles with long runs on both sides nor thin matrices with beta; the autotuner's mirror of the rule says
+    the same."""
+    _torch()
+    from ttc_b200 import Plan
+    from ttc_b200.autotune import Problem, staged_claims
+    plan = Plan(perm, size, dtype, beta != 0)
+    d = plan.describe()
+    assert (d["tile"]["claims"], d["tile"]["claim_group"]) == (claims, group), d
+    assert staged_claims(Problem(perm, size, dtype, 1.0, beta), {}, d) == bool(claims), d
+    plan.close()
+
+
 @pytest.mark.parametrize("group", [7, 8, 9, 12, 13, 16, 63, 64, 100])
 def test_claims_of_any_group_size(group):
     """Claims of up to 64 consecutive tiles (more count as 64), decoded in batches of the largest divisor up to

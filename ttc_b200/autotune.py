@@ -146,9 +146,10 @@ def schedule_alternatives(p: Problem, desc: dict, k: int) -> list[dict]:
 
 def staged_claims(p: Problem, tuning: dict, desc: dict) -> bool:
     """Whether the staged kernel claims tiles from counters under this schedule: asked for
-    (round_robin -1), or the planner's rule for round_robin 0 - a call that moves 128 MB or more (150 MB
-    when B is read back) with 8 or more tiles per CTA (CTAs estimated as SMs x the schedule's CTAs per SM, else as
-    many as the ring's shared memory lets share an SM)."""
+    (round_robin -1), or the planner's rule for round_robin 0 - tensors of 160 MB or more, 8 or more tiles per
+    CTA (CTAs estimated as SMs x the schedule's CTAs per SM, else as many as the ring's shared memory lets share
+    an SM), but neither tiles under 17 KiB with runs of 512 bytes or more on both sides (and wider than 4-byte
+    accesses on A) nor, with beta, long runs of 16-byte accesses on A against 4-byte accesses on B."""
     rr = tuning.get("round_robin", 0)
     if rr != 0:
         return rr == -1
@@ -162,7 +163,13 @@ def staged_claims(p: Problem, tuning: dict, desc: dict) -> bool:
         S = tuning.get("stages") or t.get("stages") or 3
         c = max(1, min(4, int(227 * 1024 // (S * stage + 3 * 1024))))
     ctas = tuning.get("blocks") or c * SMS
-    return p.bytes() >= (150_000_000 if p.beta_nonzero else 128_000_000) and t.get("ntiles", 0) >= 8 * ctas
+    ea, eb = ELEM_BYTES[ta], ELEM_BYTES[tb]
+    if p.elements() * (ea + eb) < 160_000_000 or t.get("ntiles", 0) < 8 * ctas:
+        return False
+    tile_bytes, run_a, run_b = t["P"] * (ea + eb * (2 if p.beta_nonzero else 1)), t["LA"] * ea, t["LB"] * eb
+    if tile_bytes < 17 * 1024 and run_a >= 512 and run_b >= 512 and desc["vecA"] * ea > 4:
+        return False
+    return not (p.beta_nonzero and desc["vecA"] * ea == 16 and desc["vecB"] * eb == 4 and run_a >= 512)
 
 
 def fused_groups(p: Problem):

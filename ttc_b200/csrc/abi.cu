@@ -128,10 +128,29 @@ using ttcb::needs_large_smem;
 // for it with round_robin = -1, or the planner's rule below); otherwise it takes the round-robin
 // order.
 static bool uses_claims(const ttcb_plan* p) { return p->claim_words != nullptr; }
-static constexpr int64_t kClaimMinBytes = 128 * 1000 * 1000, kClaimMinBytesBeta = 150 * 1000 * 1000;
+// The planner's rule for claims. CTAs that drift apart under the round-robin order read lines of A, and write parts
+// of lines of B, that their neighbours have left behind; claims keep them together and cost each tile a share
+// of a round trip. From 457 plans timed under both orders, back to back on buffers that no cache holds:
+// * the tensors exceed the 126 MB L2 by a quarter: of 128 smaller problems claims took 0.91-1.47 of the
+//   round-robin order's time, 1.05 on average, of 329 larger ones under these rules 0.65-1.11, 0.94 on average;
+// * two tiles per claim; four of tiles under 13 KiB, whose claim would not be back in time (0.94 of a pair's time
+//   on average, 1.02 for larger tiles; one tile per claim 1.03);
+// * no claims for tiles under 17 KiB whose runs are 512 bytes or more on both sides, so that neighbours share few
+//   lines, unless 4-byte accesses on A say that rows start anywhere: 0.92-1.13, 1.05 on average (the other tiles
+//   under 17 KiB 0.65-1.11, 0.955 on average);
+// * nor for thin matrices with beta, long runs of 16-byte accesses on A against 4-byte accesses on B, which are
+//   bound by instructions: 0.99-1.02 (27 x 1941807: 140.4 against 136.9 us).
+static constexpr int64_t kClaimMinFootprint = 160 * 1000 * 1000;
 static constexpr int kClaimMinTilesPerCta = 8;
-static constexpr int64_t kClaimPairTileBytes = 13 * 1024;
-static constexpr int64_t kClaimSingleTileBytes = 20 * 1024;
+static constexpr int64_t kClaimPairTileBytes = 13 * 1024, kClaimAnyRunTileBytes = 17 * 1024;
+static constexpr int64_t kClaimLongRun = 512;
+static bool planner_claims(const ttcb_plan* p, const TileDesc* td, int64_t tile_bytes) {
+  const int64_t EA = dtype_bytes(p->ta), EB = dtype_bytes(p->tb), runA = td->LA * EA, runB = td->LB * EB;
+  if (p->N * (EA + EB) < kClaimMinFootprint || td->nfull < (int64_t)kClaimMinTilesPerCta * p->blocks_async) return false;
+  if (tile_bytes < kClaimAnyRunTileBytes && runA >= kClaimLongRun && runB >= kClaimLongRun && p->vecA * EA > 4)
+    return false;
+  return !(p->beta_nonzero && p->vecA * EA == 16 && p->vecB * EB == 4 && runA >= kClaimLongRun);
+}
 // The staged kernel moves A runs with bulk copies when the plan's layout allows it and A's pointer
 // meets the layout's alignment (shifted runs take any pointer; plain runs need the 16-byte vector).
 static bool uses_bulk(const ttcb_plan* p, const TileDesc* td, int va, int EA) {
@@ -203,34 +222,16 @@ static ttcb_status plan_finish_device(ttcb_plan* p) {
       if (s != TTCB_OK) return s;
     }
     if (td->async_ok) {
-      // Tiles are claimed in order from counters when the schedule asks for it, or by default for
-      // calls that move 128 MB or more (150 MB when B is read too; the L2 holds 126 MB) with 8 tiles or
-      // more per CTA. Past L2, the
-      // CTAs' drift apart under the round-robin order spreads the tiles in motion over A and B: back to
-      // back over the 200 MiB sweep, claims against round robin took 0.78-0.97 of the time on 52 of the
-      // 61 tile plans and 1.00-1.06 on the others (tiles of 7-11 KiB), the sweep 6.24 against 6.62 ms; 156 MB
-      // (11 tiles of 48 KiB per CTA) 27.7 against 31.3 us. Within L2 the order does not matter and the claims
-      // cost (51 MB in tiles of 8 KiB: 15.5 against 12.2 us; 93 MB: 18.9 against 18.3; 147 MB with B read
-      // back, 98 MB of tensors: 27.0 against 26.5).
+      // tiles are claimed in order from counters when the schedule asks for it, or by the planner's rule
       const int EA = dtype_bytes(p->ta);
       const int64_t tiles = (int64_t)td->nfull + (p->rag_inline ? (int64_t)td->nrag0 + td->nrag1 : 0);
       s = grid_for(staged_kernel_id(p, td, td->reg_ok, false), p->smem_async, &p->blocks_async, tiles);
       if (s != TTCB_OK) return s;
-      const int64_t elem_bytes = EA + dtype_bytes(p->tb) * (p->beta_nonzero ? 2 : 1);
-      const bool claims_by_default = p->tuning.round_robin == 0 && p->N * elem_bytes >= (p->beta_nonzero ? kClaimMinBytesBeta : kClaimMinBytes) &&
-                                     td->nfull >= (int64_t)kClaimMinTilesPerCta * p->blocks_async;
-      // Tiles per claim: four of tiles under 13 KiB, whose claim would not be back in time (back to back
-      // over the sweep, four against two: 0.88-0.99 of the time for tiles of 6-12 KiB, 1.01-1.08 for tiles
-      // of 14 KiB and more), else two; but one of tiles of 20 KiB and more in a three-stage ring whose B
-      // runs are at most 160 bytes, so that neighbours, which share lines or DRAM bursts of B, are
-      // written by different CTAs at the same time (one against two on 10 such shapes of 200 MiB: 0.89-1.01
-      // of the time; with longer runs or deeper rings 1.00-1.17). Of 64-byte runs a pair fills a line:
-      // two again (fp64 with beta, 99.8 against 104.8 us and 91.4 against 100.7).
-      const int64_t tile_bytes = td->P * elem_bytes;
-      const int64_t b_run = td->LB * (int64_t)dtype_bytes(p->tb);
-      const bool short_b = tile_bytes >= kClaimSingleTileBytes && td->nstages == 3 && b_run <= 160 && b_run != 64;
-      const int group = tile_bytes < kClaimPairTileBytes ? 4 : short_b ? 1 : 2;
-      p->claim_group = p->tuning.claim_group > 0 ? std::min(p->tuning.claim_group, ttcb::kMaxClaimGroup) : group;
+      const int EB = dtype_bytes(p->tb);
+      const int64_t tile_bytes = td->P * (int64_t)(EA + EB * (p->beta_nonzero ? 2 : 1));
+      const bool claims_by_default = p->tuning.round_robin == 0 && planner_claims(p, td, tile_bytes);
+      p->claim_group = p->tuning.claim_group > 0 ? std::min(p->tuning.claim_group, ttcb::kMaxClaimGroup)
+                       : tile_bytes < kClaimPairTileBytes ? 4 : 2;
       if (p->tuning.round_robin == -1 || claims_by_default) {
         e = cudaMalloc(&p->claim_words, sizeof(unsigned int) * 2 * ttcb::kClaimSlots);
         if (e != cudaSuccess) {
