@@ -476,9 +476,9 @@ static constexpr double kTargetInFlightBytes = 18.0 * 1024 * 1024;
 // three and 12% with two, although single cases repeated alone ran faster with them) and picks the
 // S in 3..6 whose W comes nearest 18 MiB, among the rings that let two CTAs share an SM when there
 // are any: with S fixed at 3 or 4 for every case the sweep measured within 0.5% of the W rule, and for
-// single cases rings far from it lost 5-15%. With beta != 0
-// three stages become four where two CTAs of either fit (tiles of 33-41 KiB): under claims of two tiles
-// 0.84-1.00 of the time of three stages on 7 shapes of 200 MiB. Problems too small to
+// single cases rings far from it lost 5-15%. (Four stages in place of three where two CTAs of either fit, tiles
+// of 33-41 KiB with beta: 0.95-1.01 of the time on 18 shapes whose tiles are claimed, 0.99-1.11 on 24 under
+// the round-robin order, which those of up to 160 MB take; not kept.) Problems too small to
 // fill the GPU twice keep the earlier rule (four stages while four CTAs fit, else three).
 // smem_for(S) is the dynamic shared memory of an S-stage ring; fixed_S (3..kMaxStages, else 0) is a
 // schedule's explicit ring depth.
@@ -516,11 +516,6 @@ static StageChoice choose_stages(int64_t P, int EA, int EB, bool beta, int vecA,
       bc = cmax;
     }
   }
-  auto ctas = [&](int S) {
-    return smem_for(S) > 200 * 1024 ? 0
-                                    : (int)((227 * 1024) / (smem_for(S) + (int64_t)ttcb::kAsyncStaticSmem + 1024));
-  };
-  if (beta && bS == 3 && !fixed && ctas(3) == 2 && ctas(4) == 2) bS = 4;
   if (bS && nfull >= 2LL * 4 * kPlanSMs) out.S = bS;
   if (fixed) out.S = fixed_S;
   return out;
