@@ -486,6 +486,7 @@ def test_tiles_of_eight_accesses_keep_access_widths_and_ragged_tiles(perm, size,
     t = j["tile"]
     assert j["vecA"] >= vec[0] and j["vecB"] >= vec[1] and t["ragged_tiles"] <= ragged, j
     assert (t["reg"] == 1 and max(t["P"] // j["vecA"], t["P"] // j["vecB"]) > 1024) == wide, j
+    assert t["reg_accesses"] == (8 if wide else 4 if t["reg"] else 0), j  # the staged kernel's form
 
 
 def test_ragged_tiles_moved_by_vectors_have_whole_vectors():

@@ -753,7 +753,8 @@ __device__ __noinline__ void ragged_pass(const TileDesc& d, const unsigned char*
 // the store phase, with a time limit. A wait that runs out adds 1 to *wait_status, waits (bounded
 // again) for the copies of the other tiles in flight and ends the CTA's loop, so that the host
 // learns of it and the context stays usable.
-template <typename TA, typename TB, int VA, int VB, bool BETA, bool STREAM, bool REG, bool DYN, bool BULK>
+// EIGHT: the register path holds reg_vecs accesses per thread and side, else kRegVec.
+template <typename TA, typename TB, int VA, int VB, bool BETA, bool STREAM, bool REG, bool DYN, bool BULK, bool EIGHT>
 __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB * sizeof(TB), BETA))
     tile_async_kernel(
     const TileDesc* __restrict__ desc, const TA* __restrict__ A, TB* __restrict__ B, TA alpha, TB beta,
@@ -808,7 +809,8 @@ __global__ void __launch_bounds__(kThreads, async_min_blocks(VA * sizeof(TA), VB
   const bool shift = VA * sizeof(TA) == 16 && d.shiftA;
   // A copies per tile: VA-element vectors, or with shifted runs the chunk slots of every run
   const int nvA = shift ? d.nsegA * d.shiftCM : P / VA, nvB = P / VB;
-  constexpr int NA = reg_vecs(VA * sizeof(TA), BETA), NB = reg_vecs(VB * sizeof(TB), BETA);  // register path's vectors
+  constexpr int NA = EIGHT ? reg_vecs(VA * sizeof(TA), BETA) : kRegVec;  // register path's vectors
+  constexpr int NB = EIGHT ? reg_vecs(VB * sizeof(TB), BETA) : kRegVec;
   constexpr bool kShift = VA * sizeof(TA) == 16;       // shifted runs are possible
   constexpr int kVecB = REG ? NB : kRegPos / VB;  // B vectors per thread with positions in gp
   constexpr int kGp = (kVecB * VB + 1) / 2;

@@ -53,9 +53,24 @@ using TB = float2;
 #define PAIR_BATCH_FN pick_batch_zc
 #endif
 
-template <int VA, int VB, bool BETA, bool STREAM, bool REG, bool DYN, bool BULK>
+// The staged kernel's form for eight 4-byte accesses per thread exists where there are such accesses.
+template <int VA, int VB, bool BETA, bool REG>
+constexpr bool kHasEight = REG && !BETA && (VA * sizeof(TA) == 4 || VB * sizeof(TB) == 4);
+
+template <int VA, int VB, bool BETA, bool STREAM, bool REG, bool DYN, bool BULK, bool EIGHT>
 static cudaError_t launch_async(const ttcb_plan* p, const void* A, void* B, const void* alpha, const void* beta,
                                 cudaStream_t stream, int blocks) {
+  auto allow_smem = [&](const void* func) {
+    if (needs_large_smem(p->smem_async)) allow_large_smem(func);
+  };
+  if constexpr (EIGHT) {
+    // tiles of at most four accesses take the form that holds four
+    const int P = reinterpret_cast<const TileDesc*>(p->host_desc.data())->P;
+    if (P <= VA * kThreads * kRegVec && P <= VB * kThreads * kRegVec) {
+      allow_smem(reinterpret_cast<const void*>(&tile_async_kernel<TA, TB, VA, VB, BETA, STREAM, REG, DYN, BULK, false>));
+      return launch_async<VA, VB, BETA, STREAM, REG, DYN, BULK, false>(p, A, B, alpha, beta, stream, blocks);
+    }
+  }
   TA al;
   std::memcpy(&al, alpha, sizeof(TA));
   TB be;
@@ -65,9 +80,8 @@ static cudaError_t launch_async(const ttcb_plan* p, const void* A, void* B, cons
   if constexpr (DYN) {
     sched = plan_claim_slot(p, stream);
     if (!sched) {
-      if (needs_large_smem(p->smem_async))
-        allow_large_smem(reinterpret_cast<const void*>(&tile_async_kernel<TA, TB, VA, VB, BETA, STREAM, REG, false, BULK>));
-      return launch_async<VA, VB, BETA, STREAM, REG, false, BULK>(p, A, B, alpha, beta, stream, blocks);
+      allow_smem(reinterpret_cast<const void*>(&tile_async_kernel<TA, TB, VA, VB, BETA, STREAM, REG, false, BULK, EIGHT>));
+      return launch_async<VA, VB, BETA, STREAM, REG, false, BULK, EIGHT>(p, A, B, alpha, beta, stream, blocks);
     }
   }
   // programmatic stream serialization: the kernel may start while the previous one in the stream
@@ -84,7 +98,7 @@ static cudaError_t launch_async(const ttcb_plan* p, const void* A, void* B, cons
   cfg.numAttrs = 1;
   // shifted A runs: A's pointer lies a0 elements past a 16-byte boundary
   const int a0 = (int)(((uintptr_t)A / sizeof(TA)) & (uintptr_t)(VA - 1));
-  return cudaLaunchKernelEx(&cfg, tile_async_kernel<TA, TB, VA, VB, BETA, STREAM, REG, DYN, BULK>,
+  return cudaLaunchKernelEx(&cfg, tile_async_kernel<TA, TB, VA, VB, BETA, STREAM, REG, DYN, BULK, EIGHT>,
                             reinterpret_cast<const TileDesc*>(p->dev_desc), static_cast<const TA*>(A),
                             static_cast<TB*>(B), al, be, sched, a0, BULK ? p->wait_status : nullptr,
                             (unsigned int)(p->claim_group | claim_batch(p->claim_group) << 16),
@@ -95,14 +109,17 @@ template <int VA, int VB, bool REG, bool DYN, bool BULK>
 static KernelRef async_ref(int variant) {
   KernelRef r;
   if (variant == 2) {
-    r.fn = &launch_async<VA, VB, true, false, REG, DYN, BULK>;
-    r.func = reinterpret_cast<const void*>(&tile_async_kernel<TA, TB, VA, VB, true, false, REG, DYN, BULK>);
+    constexpr bool E = kHasEight<VA, VB, true, REG>;
+    r.fn = &launch_async<VA, VB, true, false, REG, DYN, BULK, E>;
+    r.func = reinterpret_cast<const void*>(&tile_async_kernel<TA, TB, VA, VB, true, false, REG, DYN, BULK, E>);
   } else if (variant == 1) {
-    r.fn = &launch_async<VA, VB, false, true, REG, DYN, BULK>;
-    r.func = reinterpret_cast<const void*>(&tile_async_kernel<TA, TB, VA, VB, false, true, REG, DYN, BULK>);
+    constexpr bool E = kHasEight<VA, VB, false, REG>;
+    r.fn = &launch_async<VA, VB, false, true, REG, DYN, BULK, E>;
+    r.func = reinterpret_cast<const void*>(&tile_async_kernel<TA, TB, VA, VB, false, true, REG, DYN, BULK, E>);
   } else {
-    r.fn = &launch_async<VA, VB, false, false, REG, DYN, BULK>;
-    r.func = reinterpret_cast<const void*>(&tile_async_kernel<TA, TB, VA, VB, false, false, REG, DYN, BULK>);
+    constexpr bool E = kHasEight<VA, VB, false, REG>;
+    r.fn = &launch_async<VA, VB, false, false, REG, DYN, BULK, E>;
+    r.func = reinterpret_cast<const void*>(&tile_async_kernel<TA, TB, VA, VB, false, false, REG, DYN, BULK, E>);
   }
   return r;
 }

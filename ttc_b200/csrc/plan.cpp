@@ -1326,7 +1326,8 @@ std::string plan_describe_json(const ttcb_plan* p) {
       << ",\"ngrid\":" << t->ngrid << ",\"nblocked\":" << t->nblocked << ",\"pad\":" << t->pad
       << ",\"pshift\":" << t->pshift << ",\"fast\":" << t->fast << ",\"async\":" << t->async_ok
       << ",\"padA\":" << t->padA << ",\"sigmaA\":" << t->sigmaA << ",\"stages\":" << t->nstages
-      << ",\"reg\":" << t->reg_ok << ",\"smem_async\":" << p->smem_async
+      << ",\"reg\":" << t->reg_ok << ",\"reg_accesses\":"
+      << (!t->reg_ok ? 0 : t->P <= p->vecA * 1024 && t->P <= p->vecB * 1024 ? 4 : 8) << ",\"smem_async\":" << p->smem_async
       << ",\"blocks_async\":" << p->blocks_async << ",\"ctas_per_sm\":" << p->ctas_per_sm
       << ",\"shifted_runs\":" << t->shiftA << ",\"bulk\":" << t->bulkA << ",\"lane_map\":" << (t->map_log2s >= 0 ? (1 << t->map_log2s) : 0) << ",\"claims\":" << (p->claim_words ? 1 : 0) << ",\"claim_group\":" << p->claim_group
       << ",\"ragged_tiles\":" << (t->nrag0 + t->nrag1) << ",\"ragged_inline\":" << p->rag_inline << ",\"ext\":[";
