@@ -340,8 +340,8 @@ def test_edge_plans_random_ragged_problems(offset):
 
 # problems whose ragged tiles are too many for the staged kernel's own launch: one ragged dimension or two
 EDGE_PLANS = [("s", -0.5, [1, 0, 2], [131, 131, 257], 512, 2), ("d", -0.5, [3, 0, 2, 1], [37, 37, 37, 67], 0, 1),
-              ("c", 0.0, [1, 0, 2], [67, 131, 401], 256, 2), ("z", 1.2, [1, 3, 2, 0], [17, 31, 67, 41], 512, 2),
-              ("zc", 0.0, [1, 0, 2], [13, 97, 2053], 0, 1), ("sd", -0.5, [1, 0, 3, 2], [97, 31, 67, 17], 8192, 1)]
+              ("c", 0.0, [1, 0, 2, 3], [41, 13, 5, 1021], 512, 1), ("z", 1.2, [1, 0, 3, 2], [37, 7, 131, 67], 256, 1),
+              ("zc", 0.0, [1, 0, 3, 2], [37, 7, 41, 163], 256, 1), ("sd", -0.5, [1, 0, 3, 2], [97, 31, 67, 17], 8192, 1)]
 
 
 @pytest.mark.parametrize("offset", [0, 1])

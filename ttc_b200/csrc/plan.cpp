@@ -1018,12 +1018,13 @@ bool unpack_raster(const ttcb_tuning& tu, int rank, int* order) {
   return true;
 }
 
-// Bytes of tile slots (complete-tile equivalents) that the ragged tiles may occupy beyond their own
-// elements when the staged kernel moves them: about 4 us at 6 TB/s, what the fork to the edge plans'
-// side stream and the join back cost on the device.
-static constexpr double kRagInlineWasteBytes = 24e6;
-// Time of a ragged tile against a complete one, by vectors and by single elements.
-static constexpr double kRagVecFactor = 1.3, kRagScalarFactor = 4.0;
+// Bytes of tile slots that the ragged tiles may occupy beyond their own elements when the staged kernel moves
+// them, slots counted by what their accesses cost: as 16-byte ones, narrower vectors by as much more, single
+// elements four times. Of 498 problems with ragged tiles, timed both ways, the rule is within 0.1% of the better
+// way on average and 8% at worst: up to 300 ragged tiles the own launch saves 3-5 us, the fork to the edge
+// plans' side stream and the join back, and from 2400 it loses 8 us and more (11440 tiles: 124.5 against 77.5).
+static constexpr double kRagInlineWasteBytes = 48e6;
+static constexpr double kRagScalarFactor = 4.0;
 
 // How the staged kernel moves a tile plan's ragged tiles in its own launch (kRagVec / kRagScalar), or 0
 // when they are better moved by other launches or the schedule asks for those.
@@ -1046,7 +1047,8 @@ static int plan_rag_inline(const ttcb_plan* p) {
   slots = (double)nrag * t->P;
   const double valid = (double)p->N - (double)t->nfull * t->P;
   const double per = dtype_bytes(p->ta) + dtype_bytes(p->tb) * (p->beta_nonzero ? 2.0 : 1.0);
-  const double waste = (slots * (vec ? kRagVecFactor : kRagScalarFactor) - valid) * per;
+  const double width = 0.5 * (16.0 / (p->vecA * dtype_bytes(p->ta)) + 16.0 / (p->vecB * dtype_bytes(p->tb)));
+  const double waste = (slots * (vec ? width : kRagScalarFactor) - valid) * per;
   if (waste > kRagInlineWasteBytes) return 0;
   return vec ? ttcb::kRagVec : ttcb::kRagScalar;
 }
