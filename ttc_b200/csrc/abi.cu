@@ -103,21 +103,22 @@ unsigned int* plan_claim_slot(const ttcb_plan* p, cudaStream_t stream) {
 }
 
 // CTAs of a launch that begins beside its predecessor take the places of the CTAs that end, one by one. Behind
-// a launch of the same plan they fit those places exactly. Behind another plan's, CTAs of other sizes leave
-// gaps in an SM's shared memory and registers, so fewer of them fit than planned, and the others run after the
-// rest: pairs of 200 MiB plans took up to 39 us longer in turn than each by itself, the 64 plans of a sweep in
-// turn 6.45-6.57 ms (6.16-6.24 when each begins after its predecessor's last CTA). A large launch (100 MB of
-// tensors; those of 100-160 MB in turn: 933 against 953 us, of 50-100 MB 778 against 764) therefore allows it
-// only where the plan has been launched twice in a row, so that a third launch is likely (a plan of 200 MiB
-// repeated: 1.00-1.04 of the time without it, of 100-160 MB 1.02-1.14). Results do not depend on it.
+// a launch of the same kernel with as much shared memory they fit those places exactly. Behind another, CTAs
+// of other sizes leave gaps in an SM's shared memory and registers, so fewer of them fit than planned, and the
+// others run after the rest: pairs of 200 MiB plans took up to 39 us longer in turn than each by itself, the 64
+// plans of a sweep in turn 6.45-6.57 ms (6.16-6.24 when each begins after its predecessor's last CTA). A large
+// launch (100 MB of tensors; those of 100-160 MB in turn: 933 against 953 us, of 50-100 MB 778 against 764)
+// therefore allows it only where it is the second of its kind in a row, so that a third is likely (a plan of 200
+// MiB repeated: 1.00-1.04 of the time without it, of 100-160 MB 1.02-1.14). Results do not depend on it.
 static constexpr int64_t kOverlapAnyBytes = 100 * 1000 * 1000;
 
-bool plan_overlaps_next(const ttcb_plan* p, cudaStream_t stream) {
-  static std::atomic<uint64_t> launches{1};
-  const uint64_t before = launches.fetch_add(1, std::memory_order_relaxed);
-  const bool in_turn = p->last_launch.exchange(before + 1, std::memory_order_relaxed) == before;
-  const bool same_stream = p->last_stream.exchange(stream, std::memory_order_relaxed) == stream;
-  return (in_turn && same_stream) || p->N * (dtype_bytes(p->ta) + dtype_bytes(p->tb)) < kOverlapAnyBytes;
+bool launch_overlaps_next(const ttcb_plan* p, const void* func, int blocks, cudaStream_t stream) {
+  static std::atomic<uint64_t> last{0};  // what the last launch of any plan was
+  uint64_t kind = reinterpret_cast<uint64_t>(func);
+  for (uint64_t x : {(uint64_t)p->smem_async, (uint64_t)blocks, reinterpret_cast<uint64_t>(stream)})
+    kind = (kind ^ x) * 0x9e3779b97f4a7c15ull;
+  const bool again = last.exchange(kind, std::memory_order_relaxed) == kind;
+  return again || p->N * (dtype_bytes(p->ta) + dtype_bytes(p->tb)) < kOverlapAnyBytes;
 }
 }  // namespace ttcb
 

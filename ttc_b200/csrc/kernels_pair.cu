@@ -98,11 +98,12 @@ static cudaError_t launch_async(const ttcb_plan* p, const void* A, void* B, cons
   cfg.numAttrs = 1;
   // shifted A runs: A's pointer lies a0 elements past a 16-byte boundary
   const int a0 = (int)(((uintptr_t)A / sizeof(TA)) & (uintptr_t)(VA - 1));
-  return cudaLaunchKernelEx(&cfg, tile_async_kernel<TA, TB, VA, VB, BETA, STREAM, REG, DYN, BULK, EIGHT>,
-                            reinterpret_cast<const TileDesc*>(p->dev_desc), static_cast<const TA*>(A),
+  const auto kernel = &tile_async_kernel<TA, TB, VA, VB, BETA, STREAM, REG, DYN, BULK, EIGHT>;
+  const int flags =
+      p->rag_inline | (launch_overlaps_next(p, reinterpret_cast<const void*>(kernel), blocks, stream) ? kOverlapNext : 0);
+  return cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const TileDesc*>(p->dev_desc), static_cast<const TA*>(A),
                             static_cast<TB*>(B), al, be, sched, a0, BULK ? p->wait_status : nullptr,
-                            (unsigned int)(p->claim_group | claim_batch(p->claim_group) << 16),
-                            p->rag_inline | (plan_overlaps_next(p, stream) ? kOverlapNext : 0));
+                            (unsigned int)(p->claim_group | claim_batch(p->claim_group) << 16), flags);
 }
 
 template <int VA, int VB, bool REG, bool DYN, bool BULK>

@@ -29,7 +29,7 @@ constexpr int kClaimSlots = 64;
 unsigned int* plan_claim_slot(const ttcb_plan* p, cudaStream_t stream);
 
 // Whether a launch of the staged kernel lets its successor in the stream begin beside it (abi.cu: the reason).
-bool plan_overlaps_next(const ttcb_plan* p, cudaStream_t stream);
+bool launch_overlaps_next(const ttcb_plan* p, const void* func, int blocks, cudaStream_t stream);
 
 // Dynamic shared memory ceiling of every plan (the planner never exceeds it).
 constexpr int kMaxDynamicSmem = 200 * 1024;

@@ -1,6 +1,5 @@
 // Host-side plan: validation, index fusion, kernel choice and descriptor construction.
 #pragma once
-#include <atomic>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -78,9 +77,6 @@ struct ttcb_plan {
   unsigned int* claim_words = nullptr;
   int claim_group = 1;            // tiles per claim
   void* claim_streams = nullptr;  // ClaimStreams (abi.cu)
-  // the plan's last launch of the staged kernel, as counted over all plans, and its stream
-  mutable std::atomic<uint64_t> last_launch{0};
-  mutable std::atomic<void*> last_stream{nullptr};
   // staged kernel with bulk A copies: count of stage waits that ran out of time (device word, zeroed
   // at creation; read and cleared by ttcb_plan_wait_timeouts)
   unsigned int* wait_status = nullptr;
