@@ -312,10 +312,12 @@ class MLP:
 
     def step(self, grads, lr=1e-3, weight_decay=0.0):
         self.t += 1
-        pairs = list(zip(self.params, grads, self.m, self.v))  # as many tensors as there are gradients
-        if not pairs:
-            return
-        params, grads, m, v = zip(*pairs)
+        params, grads, m, v = self.params, list(grads), self.m, self.v
+        if len(grads) != len(params):  # as many tensors as there are of both
+            k = min(len(grads), len(params))
+            if not k:
+                return
+            params, grads, m, v = params[:k], grads[:k], m[:k], v[:k]
         n = (ctypes.c_int * len(params))(*[p.numel() for p in params])
         _native.check(_lib().ttcb_mlp_adam_multi(len(params), _ptrs(params), _ptrs(grads), _ptrs(m), _ptrs(v), n, lr,
                                                  0.9, 0.999, 1e-8, weight_decay, self.t, _s()))
