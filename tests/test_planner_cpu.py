@@ -489,6 +489,28 @@ def test_tiles_of_eight_accesses_keep_access_widths_and_ragged_tiles(perm, size,
     assert t["reg_accesses"] == (8 if wide else 4 if t["reg"] else 0), j  # the staged kernel's form
 
 
+def test_selector_features_know_the_register_path():
+    """The selector's feature that tells tiles on the staged kernel's register path from the others, computed
+    from shape-only plans, is the full plan's `reg`, tiles of eight 4-byte accesses per thread among them."""
+    import ttc_b200.workloads as wl
+    from ttc_b200.autotune import Problem
+    from ttc_b200.core import plan_shapes
+    from ttc_b200.cost_model import _shape_part
+    wide = 0
+    for c in wl.sweep_cases(2024) + wl.sweep_cases(77) + wl.learning_cases(11, 100):
+        beta = c["beta"] != 0
+        for tu in ({}, {"tile_elems": 2048}, {"tile_elems": 8192, "run_bytes": 256}):
+            full = plan_host_json(c["perm"], c["size"], c["dtype"], beta, None, None, tu)
+            t = full.get("tile")
+            if not t or not t["async"]:
+                continue
+            shape = plan_shapes(c["perm"], c["size"], c["dtype"], beta, None, None, [tu])[0]
+            p = Problem(c["perm"], c["size"], c["dtype"], 1.0, c["beta"])
+            assert _shape_part(p, shape)[1][2] == _shape_part(p, full)[1][2] == t["reg"], (c, tu, t)
+            wide += t["reg"] == 1 and max(t["P"] // full["vecA"], t["P"] // full["vecB"]) > 1024
+    assert wide >= 10, wide
+
+
 def test_ragged_tiles_moved_by_vectors_have_whole_vectors():
     """When the staged kernel moves ragged tiles by vectors (ragged_inline 1), every vector of a ragged
     tile is valid as a whole or not at all, in A order (vecA) and in B order (vecB), and at aligned

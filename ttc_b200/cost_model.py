@@ -85,7 +85,8 @@ def _shape_part(p: Problem, desc: dict) -> tuple:
             math.log2(max(P, 1)) / 14.0, math.log2(max(LA, 1)) / 14.0, math.log2(max(LB, 1)) / 14.0,
             desc["vecA"] / 4.0, desc["vecB"] / 4.0,
             math.log2(max(LA * ELEM_BYTES[ta], 1)) / 16.0, math.log2(max(LB * ELEM_BYTES[tb], 1)) / 16.0]
-    mid = [min(desc["est_cost"], 200.0) / 32.0, math.log2(max(nt, 1)) / 25.0, float(t.get("fast", 0))]
+    # (reg: the staged kernel holds the tile's offsets in registers)
+    mid = [min(desc["est_cost"], 200.0) / 32.0, math.log2(max(nt, 1)) / 25.0, float(t.get("reg", t.get("fast", 0)))]
     tail = [math.log2(max(P * ELEM_BYTES[ta], 1)) / 16.0,
             math.log2(max(P / max(LA, 1), 1)) / 10.0, math.log2(max(P / max(LB, 1), 1)) / 10.0]
     tile_bytes = P * (ELEM_BYTES[ta] + ELEM_BYTES[tb] * (2 if p.beta_nonzero else 1))
@@ -493,8 +494,8 @@ def load_default(path: Optional[Path] = None) -> MLP:
 # default: at least POLICY["hi"] (log GB/s), its top-1 untimed; between POLICY["lo"] and
 # POLICY["hi"], its top POLICY["k"] candidates and the default are timed and the fastest kept; below
 # POLICY["lo"] the default stays. On the 500 held-out problems' stored timings, timing the top 1, 2
-# or 3 with the default kept 0.952, 0.964 and 0.971 of the best measured GB/s (the default alone
-# 0.925). `train` fits the thresholds on its held-out problems and stores them with the model.
+# or 3 with the default kept 0.950, 0.959 and 0.964 of the best measured GB/s (the default alone
+# 0.927). `train` fits the thresholds on its held-out problems and stores them with the model.
 DEFAULT_POLICY = {"lo": 0.02, "hi": 0.3, "k": 2}  # a trained model stores its own (lo, hi, k)
 
 
@@ -690,9 +691,11 @@ def stored_selection(pred: np.ndarray, y: np.ndarray, case: np.ndarray, meta: di
             "gain_over_default": float(np.mean(gated / dflt))}
 
 
-def fit_policy(pred: np.ndarray, y: np.ndarray, case: np.ndarray, meta: dict, timing_cost: float = 0.005) -> dict:
+def fit_policy(pred: np.ndarray, y: np.ndarray, case: np.ndarray, meta: dict, timing_cost: float = 0.0075) -> dict:
     """The policy (thresholds and candidates timed) that keeps the largest share of the best GB/s on
-    these problems, less `timing_cost` per candidate timed per problem (the policy's tuning time)."""
+    these problems, less `timing_cost` per candidate timed per problem (the policy's tuning time). At
+    0.0075 a third candidate is not timed: on stored timings it adds 0.5 points, on fresh ones none (0.966 of the
+    search winner's GB/s with two and with three, three runs each), for a third more tuning time."""
     best, best_score = dict(DEFAULT_POLICY), -1e9
     for k in (1, 2, 3):
         for lo in (0.0, 0.01, 0.02, 0.05, 0.1, 0.2, float("inf")):

@@ -1337,8 +1337,12 @@ std::string plan_describe_json(const ttcb_plan* p) {
     o << "]}";
   } else if (p->kernel == TTCB_KERNEL_TILE && p->shape_only) {
     const bool fits = p->tile_P / p->vecA <= 1024 && p->tile_P / p->vecB <= 1024;
+    const int EA = dtype_bytes(p->ta), EB = dtype_bytes(p->tb);
+    const bool reg = ttcb::reg_path_fits(p->tile_P, p->vecA, EA, p->vecB, EB, p->beta_nonzero != 0) &&
+                     p->tile_P * EA < 65536 && p->tile_P * EB < 65536;
     o << ",\"tile\":{\"P\":" << p->tile_P << ",\"LA\":" << p->tile_LA << ",\"LB\":" << p->tile_LB
-      << ",\"ntiles\":" << p->tile_ntiles << ",\"fast\":" << (fits ? 1 : 0) << ",\"stages\":" << p->shape_stages
+      << ",\"ntiles\":" << p->tile_ntiles << ",\"fast\":" << (fits ? 1 : 0) << ",\"reg\":" << (reg ? 1 : 0)
+      << ",\"stages\":" << p->shape_stages
       << ",\"ctas_per_sm\":" << p->ctas_per_sm << ",\"shifted_runs\":" << (p->shape_shifted ? 1 : 0)
       << ",\"bulk\":" << (p->shape_bulk ? 1 : 0)
       << ",\"shape_only\":1,\"ext\":[";
