@@ -304,16 +304,17 @@ class MLP:
 
     def loss_grad(self, out, y):
         import torch
-        d = torch.empty_like(out)
+        d, n = torch.empty_like(out), out.numel()
         # (the library writes no loss for an empty batch: 0)
-        loss = (torch.empty if out.numel() else torch.zeros)(1, device="cuda")
-        _native.check(_lib().ttcb_mlp_mse(out.data_ptr(), y.data_ptr(), out.numel(), d.data_ptr(), loss.data_ptr(),
-                                          _s()))
+        loss = torch.empty(1, device="cuda") if n else torch.zeros(1, device="cuda")
+        _native.check(_lib().ttcb_mlp_mse(out.data_ptr(), y.data_ptr(), n, d.data_ptr(), loss.data_ptr(), _s()))
         return loss, d
 
     def step(self, grads, lr=1e-3, weight_decay=0.0):
         self.t += 1
-        params, grads, m, v = self.params, list(grads), self.m, self.v
+        params, m, v = self.params, self.m, self.v
+        if type(grads) is not list:
+            grads = list(grads)
         if len(grads) != len(params):  # as many tensors as there are of both
             k = min(len(grads), len(params))
             if not k:
