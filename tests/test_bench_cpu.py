@@ -72,3 +72,20 @@ def test_sweep_schedule_rules():
         c = cases[k]
         d = plan_host_json(c["perm"], c["size"], c["dtype"], c["beta"] != 0, tuning={"bulk_copies": 1})
         assert ss.bulk_copy_bytes(d, c["dtype"]) == want
+
+
+def test_reference_arm_never_times_the_port(monkeypatch, capsys):
+    """Without TTC's generated code for every case, the reference arm says that it is unavailable, in one line,
+    instead of timing this project's port of TTC's loop."""
+    import json
+    import types
+
+    import bench
+    import pytest
+    for covered in (0, 3):
+        monkeypatch.setattr(bench, "CpuReference", lambda cases: types.SimpleNamespace(covered=covered, total=len(cases)))
+        monkeypatch.setattr(bench, "host_inputs", lambda *a: pytest.fail("no inputs are needed"))
+        args = types.SimpleNamespace(seed=2024, cases=4, warmup=1, steps=1)
+        assert bench.run_reference_arm(args, 0, 1) == 0
+        line = json.loads(capsys.readouterr().out)
+        assert line["impl"] == "reference" and "unavailable" in line and "value" not in line
