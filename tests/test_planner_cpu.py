@@ -477,11 +477,12 @@ def test_lane_maps():
 @pytest.mark.parametrize("perm,size,vec,ragged,wide", [
     ([2, 0, 3, 1], [1254, 22, 2, 305], (2, 4), 0, False), ([1, 0, 2], [65, 17, 12981], (2, 2), 1, False),
     ([2, 1, 4, 0, 3], [897, 2, 7, 104, 17], (1, 2), 0, False), ([1, 3, 5, 2, 4, 0], [10, 31, 11, 99, 2, 78], (2, 1), 0, False),
+    ([1, 2, 3, 0], [223, 29, 121, 67], (1, 1), 3687, False), ([3, 4, 1, 0, 2], [137, 81, 15, 3, 105], (1, 1), 8505, False),
     ([1, 0], [27, 1941807], (4, 1), 1, True), ([2, 1, 0], [10, 25, 209715], (2, 1), 0, True)])
 def test_tiles_of_eight_accesses_keep_access_widths_and_ragged_tiles(perm, size, vec, ragged, wide):
     """A tile of more than four 4-byte accesses per thread is taken (fp32, beta = 0, 64 MB and more) only where
-    the accesses are as wide as those of the tile that would be taken without them, and the ragged tiles as
-    few."""
+    the accesses are as wide as those of the tile that would be taken without them, the ragged tiles as few, and
+    B's runs not cut below 64 bytes."""
     j = plan_host_json(perm, size, "s", False)
     t = j["tile"]
     assert j["vecA"] >= vec[0] and j["vecB"] >= vec[1] and t["ragged_tiles"] <= ragged, j

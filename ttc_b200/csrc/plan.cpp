@@ -387,7 +387,7 @@ static void enumerate_tiles(const FusedProblem& f, int EA, int EB, bool beta, in
 
 // The cheapest enumerated tile under the tuning's size limit and run-length preference (ties go to
 // the longer shorter run).
-static bool pick_tile(const std::vector<TileCand>& cands, int EA, const ttcb_tuning& tu, TileCand& best) {
+static bool pick_tile(const std::vector<TileCand>& cands, int EA, int EB, const ttcb_tuning& tu, TileCand& best) {
   const int64_t Pmax = tile_pmax(EA, tu);
   bool found = false;
   TileCand four;  // the cheapest when the register path holds four accesses per thread
@@ -406,11 +406,14 @@ static bool pick_tile(const std::vector<TileCand>& cands, int EA, const ttcb_tun
     found = true;
   }
   // A tile that is the cheapest by its eight accesses alone has to keep the access widths of the tile that
-  // would be taken without them and leave about as few ragged tiles. Of 25 problems of 84 to 420 MB, 17 keep
-  // both: 0.76-1.06 of the time with eight, 0.89 on average. The others took 1.00-1.23 (narrower vectors:
-  // 1254 x 22 x 2 x 305, 24.9 against 32.5 us; 6-11% of ragged tiles where there were none: 1.05-1.21).
+  // would be taken without them, leave about as few ragged tiles, and not cut B's runs below two sectors. Of 25
+  // problems of 84 to 420 MB, 17 keep the first two: 0.76-1.06 of the time with eight, 0.89 on average. The others
+  // took 1.00-1.23 (narrower vectors: 1254 x 22 x 2 x 305, 24.9 against 32.5 us; 6-11% of ragged tiles where there
+  // were none: 1.05-1.21). Of 110 more of 420 MB that keep them, 0.88 on average, two cut B's runs from 180 and 256
+  // bytes to 48 and 32: 1.38 and 1.50.
   if (found && best.cost < best.cost4 &&
-      (best.vecA < four.vecA || best.vecB < four.vecB || best.ragged > four.ragged + kWideTileRagged))
+      (best.vecA < four.vecA || best.vecB < four.vecB || best.ragged > four.ragged + kWideTileRagged ||
+       (best.LB * EB < 64 && best.LB < four.LB)))
     best = four;
   return found;
 }
@@ -446,11 +449,11 @@ static bool best_tile(const FusedProblem& f, int EA, int EB, bool beta, const tt
       c->beta = beta;
       c->vec = vec;
     }
-    return pick_tile(c->cands, EA, tu, best);
+    return pick_tile(c->cands, EA, EB, tu, best);
   }
   std::vector<TileCand> cands;
   enumerate_tiles(f, EA, EB, beta, vec, tile_pmax(EA, tu), cands);
-  return pick_tile(cands, EA, tu, best);
+  return pick_tile(cands, EA, EB, tu, best);
 }
 
 void plan_tile_cache_begin() {
